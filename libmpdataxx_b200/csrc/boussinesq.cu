@@ -56,17 +56,20 @@ struct geom {
   template <class T> __device__ __forceinline__ T rdx(int d) const { if constexpr (sizeof(T) == 4) return rdxf[d]; else return rdxd[d]; }
 };
 
-// Every interior point once: threadIdx.x runs along the last (contiguous)
-// axis, threadIdx.y and the blocks over the rows of the other axes.
+// Every interior point once: a warp takes a segment of 32 points of a row (the
+// last, contiguous axis), the warps of the grid walk over the segments.  Segments
+// rather than whole rows: a 201 x 201 grid has 201 rows, which gave 26 blocks of 8
+// warps (k_gcr_update 28 us per launch there), and 1407 segments.
 template <class F>
 __device__ __forceinline__ void for_interior(const geom &g, F &&fn) {
-  for (int row = blockIdx.x * blockDim.y + threadIdx.y; row < g.nrows; row += gridDim.x * blockDim.y) {
-    int i = row, j = 0;
-    if (g.nd == 3) { i = row / g.n[1]; j = row - i * g.n[1]; }
-    for (int f = threadIdx.x; f < g.nf; f += blockDim.x) {
-      if (g.nd == 3) fn(i, j, f);
-      else fn(i, f, 0);
-    }
+  const int nseg = (g.nf + 31) >> 5;
+  const long long tot = (long long)g.nrows * nseg;
+  for (long long q = (long long)blockIdx.x * blockDim.y + threadIdx.y; q < tot; q += (long long)gridDim.x * blockDim.y) {
+    const int row = tot <= 0x7fffffff ? int(unsigned(q) / unsigned(nseg)) : int(q / nseg);
+    const int f = int(q - (long long)row * nseg) * 32 + threadIdx.x;
+    if (f >= g.nf) continue;
+    if (g.nd == 3) { const int i = row / g.n[1]; fn(i, row - i * g.n[1], f); }
+    else fn(row, f, 0);
   }
 }
 
@@ -138,41 +141,45 @@ struct vec_u {
 template <class T> struct is_vec : std::false_type {};
 template <class T> struct is_vec<vec_u<T>> : std::true_type {};
 
-// lap_tmp[d] at interior coordinate q: grad, minus u (err_init), zero on a rigid wall (set_edges)
-template <class T, class F, class U>
-__device__ __forceinline__ T lt(const F &A, const U &u, const geom &g, int d, long long base, long long sd,
-                                long long ubase, long long usd, int q) {
-  if (rigid_edge(g, d, q)) return T(0);
-  T v = grad<T>(A, g, d, base, sd, q);
-  if constexpr (is_vec<U>::value) v -= T(u.u[d].o[ubase + q * usd]);
-  if (g.norm) v = v / g.dn<T>(d, base + q * sd);
-  return v;
-}
-// lap_tmp[d] at coordinate q in [-1, n] (its own pressure halo fill)
-template <class T, class F, class U>
-__device__ __forceinline__ T LT(const F &A, const U &u, const geom &g, int d, long long base, long long sd,
-                                long long ubase, long long usd, int q) {
-  int qa, qb;
-  pres_src(g, d, q, qa, qb);
-  T v = lt<T>(A, u, g, d, base, sd, ubase, usd, qa);
-  if (qb >= 0) v = T(2) * v - lt<T>(A, u, g, d, base, sd, ubase, usd, qb);
-  return v;
+// One side of the outer difference of lap() along an axis of n points: lap_tmp at
+// c + 1 or c - 1, with the pressure halo fill of lap_tmp itself.  lap_tmp vanishes on
+// a rigid wall (set_edges) and beyond it the fill gives 2 x 0 - (its mirror), so it is
+// always a centred difference at one coordinate q, kept, zeroed or negated, whose two
+// neighbours lie in the interior or wrap around.
+struct lap_side {
+  int q, hi, lo;
+  bool zero, neg;
+};
+__device__ __forceinline__ lap_side side_of(const geom &g, int d, int q) {
+  const int n = g.n[d];
+  const bool cl = g.bc[d][0] == MPDX_BC_CYCLIC, cr = g.bc[d][1] == MPDX_BC_CYCLIC;
+  lap_side r;
+  r.neg = (q < 0 && !cl) || (q > n - 1 && !cr);
+  if (q < 0) q = cl ? q + n - 1 : -q;
+  else if (q > n - 1) q = cr ? q - (n - 1) : 2 * (n - 1) - q;
+  r.q = q;
+  r.zero = rigid_edge(g, d, q);
+  r.hi = q + 1 <= n - 1 ? q + 1 : 1;
+  r.lo = q - 1 >= 0 ? q - 1 : n - 2;
+  return r;
 }
 // lap(A) at interior point (i, j, k): div(grad A [- u]) (mpdata_rhs_vip_prs_common.hpp:49-84,
-// nabla_formulae.hpp:184-215).  `lay` is the layout shared by A's fields.
+// nabla_formulae.hpp:184-215).  `lay` is the layout shared by A's fields.  Lanes whose
+// whole stencil is interior and lanes near a face go the same way wherever one lane of
+// the warp is near a face (no loads behind branches: the nested halo rules this
+// replaces took about twice the time); warps that are wholly inside skip the index rules.
 template <class T, class F, class U>
 __device__ __forceinline__ T lap(const F &A, const dfield<T> &lay, const U &u, const geom &g, int i, int j, int k) {
   const int c[3] = {i, j, k};
   const long long o = off3(lay, i, j, k);
   T r = T(0);
   // Points whose whole stencil (c - 2 .. c + 2 along every axis) is interior: no halo
-  // rule and no wall applies, so LT(c +- 1) = grad(c +- 1) [- u(c +- 1)] and aval is a
-  // plain read.  Same operations in the same order as the general form below.
+  // rule and no wall applies.  Same operations in the same order as the form below.
   bool inner = true;
 #pragma unroll
   for (int d = 0; d < 3; ++d)
     if (d < g.nd) inner = inner && c[d] >= 2 && c[d] <= g.n[d] - 3;
-  if (inner) {
+  if (__all_sync(__activemask(), inner)) {
     const T a0 = A(o);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -198,15 +205,20 @@ __device__ __forceinline__ T lap(const F &A, const dfield<T> &lay, const U &u, c
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     if (d >= g.nd) break;
-    const long long sd = stride(lay, d);
-    const long long base = o - c[d] * sd;
-    long long ubase = 0, usd = 0;
-    if constexpr (is_vec<U>::value) {
-      usd = stride(u.u[d], d);
-      ubase = off3(u.u[d], i, j, k) - c[d] * usd;
+    const long long sd = stride(lay, d), base = o - c[d] * sd;
+    const T dx = g.dx<T>(d), rdx = g.rdx<T>(d);
+    T v[2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const lap_side s = side_of(g, d, w == 0 ? c[d] + 1 : c[d] - 1);
+      T x = mpdx::qdiv<T>(A(base + s.hi * sd) - A(base + s.lo * sd), dx, rdx) * T(0.5);
+      if constexpr (is_vec<U>::value)
+        x -= T(u.u[d].o[off3(u.u[d], i, j, k) + (s.q - c[d]) * stride(u.u[d], d)]);
+      if (g.norm) x = x / g.dn<T>(d, base + s.q * sd);
+      x = s.zero ? T(0) : x;
+      v[w] = s.neg ? T(2) * T(0) - x : x;
     }
-    const T term = mpdx::qdiv<T>(LT<T>(A, u, g, d, base, sd, ubase, usd, c[d] + 1) - LT<T>(A, u, g, d, base, sd, ubase, usd, c[d] - 1),
-                                 g.dx<T>(d), g.rdx<T>(d)) * T(0.5);
+    const T term = mpdx::qdiv<T>(v[0] - v[1], dx, rdx) * T(0.5);
     r = d == 0 ? term : r + term;
   }
   return r;
@@ -332,7 +344,7 @@ __device__ __forceinline__ double ddv(dd a) { return a.s + a.c; }
 
 template <class T>
 __global__ void k_gcr_reset(gcr_dev<T> *dv) {
-  dv->converged = 0; dv->done = 0; dv->stuck = 0; dv->cur = 0; dv->iters = 0; dv->arrive = 0u; dv->bad = 0;
+  dv->converged = 0; dv->done = 0; dv->stuck = 0; dv->cur = 0; dv->iters = 0; dv->arrive = 0u; dv->bad = 0; dv->timeout = 0;
 }
 // after the learned corrections: plain GCR continues from the current iterate
 template <class T>
@@ -765,6 +777,367 @@ void launch_inner(int v, unsigned G, dim3 blk, cudaStream_t s, const geom &g, in
 }
 
 // ---------------------------------------------------------------------------
+// The whole GCR(k) iteration in one cooperative launch: one block per SM at most;
+// every block keeps the scalars (beta, alpha, the pending sums) for itself.  Each
+// reduction carries the barrier: a block writes its partial sums, counts itself in,
+// one thread waits until all blocks have, then every block adds all partials in
+// block order and gets the same bits.  Per-point arithmetic is that of k_gcr_update
+// and k_gcr_direction.  What bounds it: the latency of the reductions (shuffle trees
+// of compensated sums, about three trips through L2) and of one or a few points per
+// thread; so all loads of a thread's points come before their arithmetic and stores.
+// (Partial sums polled by all warps of all blocks, without the counter, were slower:
+// the polling slows the blocks that still work.)  R: points per thread held in registers from the first to the second
+// half of a step, 0: any number, read again.  For grids whose two launches per inner
+// step are latency-bound (rule and figures at loop_grid).  A wait that gives up after
+// about two seconds sets dv->timeout and leaves.
+constexpr int kLoopThreads = 512;
+
+// lap()'s index rules for every coordinate of an axis, in shared memory: element
+// offsets from the point to the neighbours of the two sides of the outer difference
+// (plus side hi, lo; minus side hi, lo),
+// and what becomes of them (lap_side).  One 16-byte read per axis and point where
+// the rules cost about 400 instructions per point.
+constexpr int kLapRows = 2048;  // coordinates of all axes together
+__device__ __forceinline__ void lap_table(const geom &g, const long long *sd, int4 *off, unsigned char *how) {
+  int base = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    if (d >= g.nd) break;
+    for (int c = threadIdx.x; c < g.n[d]; c += blockDim.x) {
+      const lap_side a = side_of(g, d, c + 1), b = side_of(g, d, c - 1);
+      const int s = int(sd[d]);
+      off[base + c] = make_int4((a.hi - c) * s, (a.lo - c) * s, (b.hi - c) * s, (b.lo - c) * s);
+      how[base + c] = (unsigned char)((a.zero ? 1 : 0) | (a.neg ? 2 : 0) | (b.zero ? 4 : 0) | (b.neg ? 8 : 0));
+    }
+    base += g.n[d];
+  }
+}
+// lap(A) at element o, coordinates c, a0 = A(o); dn: lap_side's q for normalize_vip
+template <class T, class F>
+__device__ __forceinline__ T lap_tab(const F &A, const geom &g, const long long *sd, const int4 *off, const unsigned char *how,
+                                     const int *c, int o, T a0) {
+  T r = T(0);
+  int base = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    if (d >= g.nd) break;
+    const int4 f = off[base + c[d]];
+    const unsigned h = how[base + c[d]];
+    base += g.n[d];
+    const T dx = g.dx<T>(d), rdx = g.rdx<T>(d);
+    const T ph = A(o + f.x), pl = f.y ? A(o + f.y) : a0, mh = f.z ? A(o + f.z) : a0, ml = A(o + f.w);
+    T gp = mpdx::qdiv<T>(ph - pl, dx, rdx) * T(0.5);
+    T gm = mpdx::qdiv<T>(mh - ml, dx, rdx) * T(0.5);
+    if (g.norm) {
+      gp = gp / g.dn<T>(d, o + (side_of(g, d, c[d] + 1).q - c[d]) * sd[d]);
+      gm = gm / g.dn<T>(d, o + (side_of(g, d, c[d] - 1).q - c[d]) * sd[d]);
+    }
+    if (h) {
+      if (h & 1) gp = T(0);
+      if (h & 2) gp = T(2) * T(0) - gp;
+      if (h & 4) gm = T(0);
+      if (h & 8) gm = T(2) * T(0) - gm;
+    }
+    const T term = mpdx::qdiv<T>(gp - gm, dx, rdx) * T(0.5);
+    r = d == 0 ? term : r + term;
+  }
+  return r;
+}
+
+// all blocks' arrivals counted up to `target`; false when the wait gave up
+__device__ __forceinline__ bool grid_wait(unsigned *bar, unsigned target, int *timeout) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    unsigned v;
+    long long t0 = 0;
+    ok = 1;
+    for (;;) {
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if (int(v - target) >= 0) break;
+      const long long t = clock64();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > (1LL << 32)) {
+        *reinterpret_cast<volatile int *>(timeout) = 1;
+        ok = 0;
+        break;
+      }
+    }
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// sums (and max / min) over the grid, the result in every thread of every block.
+// board: two alternating boards of [value][block] partial results; bar counts the
+// arrivals since the handle was made (epoch reductions x blocks).
+template <int NS, bool MM>
+__device__ __forceinline__ bool all_reduce(dd (&acc)[NS], int ns, double &mx, double &mn, double2 *board, unsigned *bar,
+                                           unsigned &epoch, int *timeout) {
+  __shared__ dd wsum[NS + 1][kLoopThreads / 32];
+  __shared__ dd res[NS + 1];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
+  const int nb = gridDim.x;
+  ++epoch;
+  double2 *const buf = board + size_t(epoch & 1) * kRedSlots * nb;
+#pragma unroll
+  for (int s = 0; s < NS; ++s)
+    if (s < ns) {
+      const dd v = warp_sum(acc[s]);
+      if (lane == 0) wsum[s][w] = v;
+    }
+  if constexpr (MM) {
+    warp_mm(mx, mn);
+    if (lane == 0) wsum[NS][w] = dd{mx, mn};
+  }
+  __syncthreads();
+  // warp s mod nw: value s of the block, then of the grid (value ns: the extrema)
+  auto tree = [&](dd v, int n) {
+    for (int off = 16; off > 0; off >>= 1) {
+      if (off >= n) continue;
+      const dd o{__shfl_down_sync(0xffffffffu, v.s, off), __shfl_down_sync(0xffffffffu, v.c, off)};
+      v = dd_add(v, o);
+    }
+    return v;
+  };
+  const int nv = ns + (MM ? 1 : 0);
+  for (int s = w; s < nv; s += nw) {
+    dd v;
+    if (s < ns) v = tree(lane < nw ? wsum[s][lane] : dd{0.0, 0.0}, nw);
+    else { v = lane < nw ? wsum[NS][lane] : dd{-DBL_MAX, DBL_MAX}; warp_mm(v.s, v.c); }
+    if (lane == 0) __stcg(buf + size_t(s) * nb + blockIdx.x, make_double2(v.s, v.c));
+  }
+  if (!grid_wait(bar, epoch * unsigned(nb), timeout)) return false;
+  for (int s = w; s < nv; s += nw) {
+    dd v = s < ns ? dd{0.0, 0.0} : dd{-DBL_MAX, DBL_MAX};
+    constexpr int U = 5;  // loads in flight per lane
+    for (int b0 = lane; b0 < nb; b0 += 32 * U) {
+      double2 p[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (b0 + 32 * u < nb) p[u] = __ldcg(buf + size_t(s) * nb + b0 + 32 * u);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (b0 + 32 * u < nb) {
+          if (s < ns) v = dd_add(v, dd{p[u].x, p[u].y});
+          else { v.s = fmax(v.s, p[u].x); v.c = fmin(v.c, p[u].y); }
+        }
+    }
+    __syncwarp();
+    if (s < ns) v = tree(v, nb);
+    else warp_mm(v.s, v.c);
+    if (lane == 0) res[s] = v;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < NS; ++s)
+    if (s < ns) acc[s] = res[s];
+  if constexpr (MM) { mx = res[ns].s; mn = res[ns].c; }
+  return true;
+}
+
+// inner steps v = 0 .. K-1 of up to max_bodies loop bodies
+template <class T, int K, int R>
+__global__ void __launch_bounds__(kLoopThreads, 1)
+    k_gcr_loop(geom g, T err_tol, dfield<T> phi, dfield<T> err0, dfield<T> err1, dfield<T> lap_err, dirs<T> D,
+               gcr_dev<T> *dv, double2 *board, unsigned *bar, long long max_bodies) {
+  constexpr int U = R > 0 ? R : 2;  // points per pass
+  T alpha[K], tden[K];
+#pragma unroll
+  for (int l = 0; l < K; ++l) { alpha[l] = dv->alpha[l]; tden[l] = dv->tmp_den[l]; }
+  T beta = dv->beta, pden = dv->pend_den, pnum = dv->pend_num;
+  int cur = dv->cur, converged = dv->converged, done = 0, stuck = 0;
+  long long iters = dv->iters;
+  double residual = dv->residual;
+  unsigned epoch = dv->epoch;
+  const int nthr = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+  // the points as a list with the last axis fastest, axes as (c0, c1, c2) with c0 = 0 in
+  // 2D; the points of a thread are nthr apart, so coordinates advance by constants
+  // with carries (no divisions), and offsets are 32-bit (a few million points)
+  const bool d3 = g.nd == 3;
+  const int cells = int(g.cells), n1 = d3 ? g.n[1] : g.n[0], n2 = d3 ? g.n[2] : g.n[1], n12 = n1 * n2;
+  const int s0 = d3 ? int(phi.s0) : 0, s1 = int(d3 ? phi.s1 : phi.s0);
+  auto split = [&](int q, int *c) {
+    c[0] = q / n12;
+    const int r = q - c[0] * n12;
+    c[1] = r / n2;
+    c[2] = r - c[1] * n2;
+  };
+  int dc[3], c_now[3], c_first[3];
+  split(nthr, dc);
+  split(min(first, cells - 1), c_first);
+  auto rewind = [&] {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) c_now[d] = c_first[d];
+  };
+  int co[U][3], o[U];
+  auto locate = [&](int q0) {  // the next U points (one beyond the last: the last one's values, unused)
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = q0 + u * nthr < cells;
+      co[u][0] = d3 ? (in ? c_now[0] : 0) : (in ? c_now[1] : 0);
+      co[u][1] = d3 ? (in ? c_now[1] : 0) : (in ? c_now[2] : 0);
+      co[u][2] = d3 && in ? c_now[2] : 0;
+      o[u] = in ? c_now[0] * s0 + c_now[1] * s1 + c_now[2] : 0;
+      c_now[2] += dc[2];
+      int up = c_now[2] >= n2 ? 1 : 0;
+      c_now[2] -= up ? n2 : 0;
+      c_now[1] += dc[1] + up;
+      up = c_now[1] >= n1 ? 1 : 0;
+      c_now[1] -= up ? n1 : 0;
+      c_now[0] += dc[0] + up;
+    }
+  };
+  __shared__ int4 t_off[kLapRows];
+  __shared__ unsigned char t_how[kLapRows];
+  const long long sd[3] = {phi.s0, phi.s1, phi.s2};
+  lap_table(g, sd, t_off, t_how);
+  __syncthreads();
+  rewind();
+  if (R > 0) locate(first);
+  T *const phio = phi.o, *const leo = lap_err.o;
+  T e[U], le[U], ph[U], po[U][K], lpo[U][K];
+  bool alive = true;
+  for (long long body = 0; body < max_bodies && !done && alive; ++body) {
+    for (int v = 0; v < K; ++v) {
+      const T den = pden;
+      const T b = den != T(0) ? -pnum / den : beta;  // beta keeps its value when tmp_den is 0
+      beta = b;
+      // first half: err' = err + beta lap_p_v, lap(err'), max |err'|, alpha sums
+      const T *const eao = cur ? err1.o : err0.o;
+      T *const ebo = cur ? err0.o : err1.o;
+      const T *lpv = D.lp[0].o;
+#pragma unroll
+      for (int l = 0; l < K; ++l)
+        if (l == v) { tden[l] = den; lpv = D.lp[l].o; }
+      const fld_axpy<T> enew{eao, lpv, b};
+      dd acc[K];
+#pragma unroll
+      for (int l = 0; l < K; ++l) acc[l] = dd{0.0, 0.0};
+      double mx = -DBL_MAX, mn = DBL_MAX;
+      if (R == 0) rewind();
+      for (int q0 = first; q0 < cells; q0 += U * nthr) {
+        if (R == 0) locate(q0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          e[u] = enew(o[u]);
+          if (R > 0) ph[u] = phio[o[u]];
+#pragma unroll
+          for (int l = 0; l < K; ++l)
+            if (l <= v) {
+              lpo[u][l] = D.lp[l].o[o[u]];
+              if (R > 0) po[u][l] = D.p[l].o[o[u]];
+            }
+          le[u] = lap_tab<T>(enew, g, sd, t_off, t_how, co[u], o[u], e[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (q0 + u * nthr >= cells) continue;
+          ebo[o[u]] = e[u];
+          if (R == 0) leo[o[u]] = le[u];
+          mx = fmax(mx, double(e[u]));
+          mn = fmin(mn, double(e[u]));
+#pragma unroll
+          for (int l = 0; l < K; ++l)
+            if (l <= v) acc[l] = dd_add(acc[l], dd{double(T(le[u] * lpo[u][l])), 0.0});
+        }
+        if (R > 0) break;
+      }
+      if (!all_reduce<K, true>(acc, v + 1, mx, mn, board, bar, epoch, &dv->timeout)) { alive = false; break; }
+      const T amx = fabs(T(mx)), amn = fabs(T(mn));
+      const T error = amx < amn ? amn : amx;  // std::max(|max|, |min|)
+      residual = double(error);
+      if (error <= err_tol) converged = 1;
+#pragma unroll
+      for (int l = 0; l < K; ++l)
+        if (l <= v && tden[l] != T(0)) alpha[l] = -T(ddv(acc[l])) / tden[l];
+      // second half: Phi += beta p_v, next direction and its lap, beta sums
+      const bool restart = v == K - 1;
+      T *pd = D.p[0].o, *lpd = D.lp[0].o;
+#pragma unroll
+      for (int l = 1; l < K; ++l)
+        if (!restart && l == v + 1) { pd = D.p[l].o; lpd = D.lp[l].o; }
+      dd bs[2] = {{0.0, 0.0}, {0.0, 0.0}};
+      if (R == 0) rewind();
+      for (int q0 = first; q0 < cells; q0 += U * nthr) {
+        if (R == 0) {
+          locate(q0);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            e[u] = ebo[o[u]];
+            le[u] = leo[o[u]];
+            ph[u] = phio[o[u]];
+#pragma unroll
+            for (int l = 0; l < K; ++l)
+              if (l <= v) { po[u][l] = D.p[l].o[o[u]]; lpo[u][l] = D.lp[l].o[o[u]]; }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (q0 + u * nthr >= cells) continue;
+          T pn = e[u], ln = le[u];
+#pragma unroll
+          for (int l = 0; l < K; ++l)
+            if (l <= v) {
+              pn = pn + alpha[l] * po[u][l];
+              ln = ln + alpha[l] * lpo[u][l];
+              if (l == v) phio[o[u]] = ph[u] + b * po[u][l];
+            }
+          pd[o[u]] = pn;
+          lpd[o[u]] = ln;
+          bs[0] = dd_add(bs[0], dd{double(T(ln * ln)), 0.0});
+          bs[1] = dd_add(bs[1], dd{double(T(e[u] * ln)), 0.0});
+        }
+        if (R > 0) break;
+      }
+      double z0 = 0, z1 = 0;
+      if (!all_reduce<2, false>(bs, 2, z0, z1, board, bar, epoch, &dv->timeout)) { alive = false; break; }
+      pden = T(ddv(bs[0]));
+      pnum = T(ddv(bs[1]));
+      cur = 1 - cur;
+    }
+    if (!alive) break;
+    iters += 1;  // end of one loop body (mpdata_rhs_vip_prs_common.hpp:111-125)
+    if (converged) done = 1;
+    if (iters > 10000) { stuck = 1; done = 1; }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+#pragma unroll
+    for (int l = 0; l < K; ++l) { dv->alpha[l] = alpha[l]; dv->tmp_den[l] = tden[l]; }
+    dv->beta = beta; dv->pend_den = pden; dv->pend_num = pnum;
+    dv->cur = cur; dv->converged = converged; dv->done = done; dv->stuck = stuck;
+    dv->iters = iters; dv->residual = residual; dv->epoch = epoch;
+  }
+}
+
+template <class T, int K>
+void launch_loop_k(int blocks, int threads, cudaStream_t s, geom g, T err_tol, dfield<T> phi, dfield<T> e0, dfield<T> e1,
+                   dfield<T> le, dirs<T> D, gcr_dev<T> *dv, double2 *board, unsigned *bar, long long max_bodies) {
+  void *args[] = {&g, &err_tol, &phi, &e0, &e1, &le, &D, &dv, &board, &bar, &max_bodies};
+  const bool one = (long long)blocks * threads >= g.cells;
+  const void *f = one ? reinterpret_cast<const void *>(k_gcr_loop<T, K, 1>) : reinterpret_cast<const void *>(k_gcr_loop<T, K, 0>);
+  MPDX_CUDA(cudaLaunchCooperativeKernel(f, dim3(blocks), dim3(threads), args, 0, s));
+}
+template <class T>
+void launch_loop(int kk, int blocks, int threads, cudaStream_t s, const geom &g, T err_tol, dfield<T> phi, dfield<T> e0,
+                 dfield<T> e1, dfield<T> le, const dirs<T> &D, gcr_dev<T> *dv, double2 *board, unsigned *bar, long long max_bodies) {
+#define MPDX_LOOP(K) launch_loop_k<T, K>(blocks, threads, s, g, err_tol, phi, e0, e1, le, D, dv, board, bar, max_bodies)
+  switch (kk) {
+    case 1: MPDX_LOOP(1); break;
+    case 2: MPDX_LOOP(2); break;
+    case 3: MPDX_LOOP(3); break;
+    case 4: MPDX_LOOP(4); break;
+    case 5: MPDX_LOOP(5); break;
+    case 6: MPDX_LOOP(6); break;
+    case 7: MPDX_LOOP(7); break;
+    default: MPDX_LOOP(8); break;
+  }
+#undef MPDX_LOOP
+}
+
+// ---------------------------------------------------------------------------
 // Learned corrections before plain GCR: q = M(err) from the network, a step along
 // q, and err updated with the exact lap of q, so the stopping test of the plain
 // iterations that follow is the reference's.  The error is updated in place (no
@@ -1188,8 +1561,27 @@ bq::geom make_geom(const mpdata_state<T> &st, const double *dijk) {
 }
 const dim3 kBlk(32, kRedThreads / 32);  // 32 points along the contiguous axis x 8 rows
 unsigned red_grid(const bq::geom &g) {
-  const long long b = (g.nrows + kBlk.y - 1) / kBlk.y;
+  const long long segs = (long long)g.nrows * ((g.nf + 31) / 32), b = (segs + kBlk.y - 1) / kBlk.y;
   return unsigned(std::max(1LL, std::min<long long>(b, kRedBlocks)));
+}
+// Blocks and threads of the one-launch GCR loop, or 0 blocks where the two kernels
+// per inner step are taken instead: grids of more than kLoopCells points, where the
+// shared planes of k_gcr_update3 save more than the launches cost, and axes that do
+// not fit the table of index rules.  FP64, us per iteration of cr, two launches
+// against one: 48 x 48 19 and 7.0, 201 x 201 22 (38 with whole rows per warp) and 7.7,
+// 400 x 400 32 and 11.6, 1000 x 1000 56 and 26, 97 x 89 x 65 53 and 22, 128 x 128 x 96
+// 67 and 47, 160 x 160 x 96 (2.46 M points) 89 and 80; gcrk with k = 3 at 97 x 89 x 65
+// 178 and 87 per body.  512 threads with 128 registers and two points per pass: with
+// 1024 threads and 64 registers fewer loads are in flight (160 x 160 x 96: 120).
+struct loop_shape {
+  int blocks, threads;
+};
+constexpr long long kLoopCells = 2500000;
+loop_shape loop_grid(const bq::geom &g, int n_sm) {
+  if (n_sm <= 0 || g.cells > kLoopCells || g.n[0] + g.n[1] + (g.nd == 3 ? g.n[2] : 0) > bq::kLapRows) return {0, 0};
+  const long long per_sm = (g.cells + n_sm - 1) / n_sm;
+  const int threads = int(std::min<long long>(bq::kLoopThreads, std::max<long long>(128, (per_sm + 31) / 32 * 32)));
+  return {int(std::min<long long>(n_sm, (g.cells + threads - 1) / threads)), threads};
 }
 }  // namespace
 
@@ -1249,6 +1641,14 @@ boussinesq<T, P>::boussinesq(const mpdx_config &c, cudaStream_t s) {
   MPDX_CUDA(cudaMemcpy(dev, &init, sizeof(init), cudaMemcpyHostToDevice));
   MPDX_CUDA(cudaMalloc(&part, sizeof(double) * kRedBlocks * kRedSlots * 2));
   MPDX_CUDA(cudaMalloc(&scratch, 64));
+  int device = 0, coop = 0;
+  MPDX_CUDA(cudaGetDevice(&device));
+  MPDX_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+  if (coop) {
+    MPDX_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, device));
+    MPDX_CUDA(cudaMalloc(&board, board_bytes()));
+    MPDX_CUDA(cudaMemset(board, 0, board_bytes()));
+  }
   MPDX_CUDA(cudaMalloc(&vip_dev, 3 * sizeof(int)));
   MPDX_CUDA(cudaMemcpy(vip_dev, vip, 3 * sizeof(int), cudaMemcpyHostToDevice));
 }
@@ -1259,6 +1659,7 @@ boussinesq<T, P>::~boussinesq() {
   if (hdev) cudaFreeHost(hdev);
   if (part) cudaFree(part);
   if (scratch) cudaFree(scratch);
+  if (board) cudaFree(board);
   if (vip_dev) cudaFree(vip_dev);
   for (float *p : {pairs, tr_r, tr_t, tr_q, tr_z, tr_dq, tr_a, tr_b}) if (p) cudaFree(p);
   if (tr_loss) cudaFree(tr_loss);
@@ -1329,18 +1730,32 @@ void boussinesq<T, P>::pressure_solve(bool simple) {
   }
   bq::k_gcr_init<P><<<G, kBlk, 0, s>>>(gm, err[0].v, p_err[0].v, lap_p_err[0].v, dev, part);
   MPDX_LAUNCH_CHECK();
+  const loop_shape loop = loop_grid(gm, n_sm);
   long long launched = 0;
   for (;;) {
     long long batch = launched == 0 ? std::max(1LL, predicted) : std::max(4LL, predicted / 4);
     if (rec) batch = std::min(batch, 16LL);  // snapshots are taken between batches
-    for (long long b = 0; b < batch; ++b)
-      for (int v = 0; v < k_iters; ++v)
-        bq::launch_inner<P>(v, G, kBlk, s, gm, k_iters, err_tol, Phi.v, err[0].v, err[1].v, lap_err.v, D, dev, part);
+    if (loop.blocks > 0) {
+      // the loop leaves by itself when it has converged; it is cut short where the
+      // host looks at the state in between (snapshots, the limit of a learned solve)
+      if (!rec) batch = learned && !restarted ? std::max(1LL, 4 * last_plain_iters + 201 - launched) : 20000;
+      bq::launch_loop<P>(k_iters, loop.blocks, loop.threads, s, gm, err_tol, Phi.v, err[0].v, err[1].v, lap_err.v, D, dev,
+                         board, board_bar(), batch);
+    } else {
+      for (long long b = 0; b < batch; ++b)
+        for (int v = 0; v < k_iters; ++v)
+          bq::launch_inner<P>(v, G, kBlk, s, gm, k_iters, err_tol, Phi.v, err[0].v, err[1].v, lap_err.v, D, dev, part);
+    }
     MPDX_LAUNCH_CHECK();
     launched += batch;
     MPDX_CUDA(cudaEventRecord(ev_solve[1], s));
     MPDX_CUDA(cudaMemcpyAsync(hdev, dev, sizeof(gcr_dev<P>), cudaMemcpyDeviceToHost, s));
     MPDX_CUDA(cudaStreamSynchronize(s));
+    if (hdev->timeout) {
+      MPDX_CUDA(cudaMemsetAsync(board, 0, board_bytes(), s));
+      MPDX_CUDA(cudaMemsetAsync(&dev->epoch, 0, sizeof(dev->epoch), s));
+      throw error(MPDX_E_TIMEOUT, "a wait of the pressure solver's blocks for one another gave up");
+    }
     // a learned solve that, after handing over, still runs far past a plain solve's
     // iteration count is redone from its start with plain GCR alone, so the learned
     // form never gives a worse result than the method without it

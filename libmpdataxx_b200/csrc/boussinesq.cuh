@@ -32,6 +32,8 @@ struct gcr_dev {
   T mean;                // ini_pressure: mean of Phi
   double residual;       // max|err| at the last convergence check
   int converged, done, stuck, cur;
+  int timeout;           // a wait of the one-launch loop gave up
+  unsigned epoch;        // reductions of the one-launch loop so far
   int bad;               // a learned direction gave non-finite sums: nothing was updated with it
   long long iters;
   unsigned int arrive;   // last-block ticket of the running reduction
@@ -64,6 +66,10 @@ struct boussinesq {
   gcr_dev<P> *hdev = nullptr;  // pinned host copy for the convergence read-back
   double *part = nullptr;      // per-block partial results of the running reduction
   double *scratch = nullptr;
+  double2 *board = nullptr;    // partial sums of the one-launch loop's blocks, then the arrival counter
+  int n_sm = 0;                // SMs (0: no cooperative launch)
+  size_t board_bytes() const { return size_t(2) * kRedSlots * n_sm * sizeof(double2) + 128; }
+  unsigned *board_bar() const { return reinterpret_cast<unsigned *>(board + size_t(2) * kRedSlots * n_sm) + 16; }
   int *vip_dev = nullptr;      // vip[] on the device
 
   // learned preconditioner (FP64 pressure solve only): the network, whether GCR
