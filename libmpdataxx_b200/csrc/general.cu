@@ -1142,6 +1142,11 @@ void general<T>::init_g() {
 template <class T>
 void general<T>::step() {
   auto &S = *s;
+  if (stage_engine<T>::covers(S)) {
+    // upwind-only step every upwind_filter_freq steps (mpdata_osc_2d.hpp:176-179)
+    stages.step(S, S.upwind_filter_freq > 0 && S.timestep % S.upwind_filter_freq == 0);
+    return;
+  }
   for (int e = 0; e < S.n_eqns; ++e) {
     xchng_sclr(S.psi[e][S.tl[e]], S.H);  // solve_loop_body: xchng(e)
     if (S.nd == 1) advop_nd<1>(e);

@@ -1,7 +1,7 @@
 // Reference-structured MPDATA path (declarations; kernels in general.cu).
 #pragma once
 
-#include "state.cuh"
+#include "stages.cuh"
 
 namespace mpdx {
 
@@ -41,6 +41,7 @@ struct general {
   bool any_rigid() const;
 
  private:
+  stage_engine<T> stages;  // the common options in a few launches per step
   int cur_e = 0;  // equation whose advop is running (the divergence form reads its other time level)
   field<T> *GC_unco(int iter);
   field<T> *GC_corr(int iter);

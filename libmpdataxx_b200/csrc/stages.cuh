@@ -1,0 +1,30 @@
+// MPDATA step in a few launches under any boundary condition (declarations;
+// kernels in stages_impl.cuh, instantiated per real type in stages_f32.cu and
+// stages_f64.cu).
+#pragma once
+
+#include "state.cuh"
+
+namespace mpdx {
+
+constexpr int kStageEqns = 4;  // equations advanced by one launch
+
+template <class T>
+struct stage_engine {
+  // work arrays of the equations after the first, where one launch takes several
+  // (the first uses the state's own)
+  struct work {
+    field<T> tmp0[3], tmp1[3], beta_up, beta_dn, psi_min, psi_max;
+  };
+  std::vector<work> more;
+
+  // whether step() covers the configuration
+  static bool covers(const mpdata_state<T> &st);
+  // advances every equation by one step; `upwind_only`: the first pass alone
+  void step(mpdata_state<T> &st, bool upwind_only);
+};
+
+extern template struct stage_engine<float>;
+extern template struct stage_engine<double>;
+
+}  // namespace mpdx

@@ -1,0 +1,615 @@
+// MPDATA step in a few launches under any boundary condition.
+//
+// The reference-structured path (general.cu) runs one kernel per formula and per
+// halo fill: about 47 launches for a 2D step with FCT and open boundaries, 70 in
+// 3D, each reading and writing whole arrays.  Here a step of n_iters passes is
+//   k_upwind    psi1 = donor-cell(psi, GC)                    (mpdata_osc_{1,2,3}d.hpp)
+// and for every corrective pass
+//   k_antidiff  all components of the antidiffusive velocity  (formulae_mpdata_{1,2,3}d.hpp)
+//   k_betas     FCT limiters of every cell, psi_min / psi_max in place
+//               (formulae_mpdata_fct_{1,2,3}d.hpp, mpdata_fct_{1,2,3}d.hpp)
+//   k_correct   limited velocities, their fluxes and the donor-cell sum
+// with the arithmetic of general.cu's functors, in their order (compiled without
+// FMA contraction: the same bits).  No kernel fills halos: a point outside the
+// domain is read where its fill would have copied it from (scalars: cyclic wrap,
+// open edge value, rigid mirror; antidiffusive velocities: the fills of
+// solver_{1,2,3}d.hpp xchng_vctr_alng(.., ad) and xchng_vctr_nrml(.., 0)).  Only the
+// advector keeps its halo in memory, filled once by general<T>::ante_loop.
+//
+// What bounds it: small grids, the launches (about 2.5 us each); large grids, the
+// traffic between the stages, 26 fields per step with FCT, in cache below about
+// 100 MB.  One thread per point of the interior, the last axis along the warp; the
+// faces at -1 and the limiter's cells just outside the domain are further blocks of
+// the same launch, so that the interior stays aligned.
+#pragma once
+
+#include <algorithm>
+#include <cfloat>
+#include <type_traits>
+
+#include "stages.cuh"
+
+namespace mpdx {
+namespace sg {
+
+template <class T> struct lim;
+template <> struct lim<float> {
+  __device__ static float tiny() { return FLT_MIN; }
+  __device__ static float eps() { return FLT_EPSILON; }
+};
+template <> struct lim<double> {
+  __device__ static double tiny() { return DBL_MIN; }
+  __device__ static double eps() { return DBL_EPSILON; }
+};
+template <class T> __device__ __forceinline__ T pos(T x) { return T(0) < x ? x : T(0); }  // std::max(0, x)
+template <class T> __device__ __forceinline__ T neg(T x) { return x < T(0) ? x : T(0); }  // std::min(0, x)
+template <class T> __device__ __forceinline__ T dmax(T a, T b) { return a < b ? b : a; }  // std::max
+template <class T> __device__ __forceinline__ T dmin(T a, T b) { return b < a ? b : a; }  // std::min
+template <class T> __device__ __forceinline__ T flux(T c, T l, T r) { return pos(c) * l + neg(c) * r; }
+
+// x / 3 and x / 6, correctly rounded without a division (mpdx::qdiv)
+template <class T> __device__ __forceinline__ T div3(T x) { return qdiv<T>(x, T(3), T(1) / T(3)); }
+template <class T> __device__ __forceinline__ T div6(T x) { return qdiv<T>(x, T(6), T(1) / T(6)); }
+
+// a field by 32-bit element strides
+template <class T>
+struct arr {
+  T *o;
+  int s0, s1;  // strides of axes 0 and 1 (the last axis: 1)
+};
+
+template <class T>
+struct eqn {
+  arr<T> in, out;             // psi of the pass, its result
+  arr<T> psin;                // psi of the step's start (k_betas)
+  arr<T> corr[3], unco[3];    // antidiffusive velocity, advector it corrects
+  arr<T> bu, bd, mn, mx;
+};
+template <class T>
+struct args {
+  eqn<T> e[kStageEqns];
+  int n[3], bc[3][2];
+  int plane;  // points of the last two axes (3D) or of the grid
+};
+
+template <int V> struct ic { static constexpr int value = V; };
+
+// ---- coordinates ----
+template <int ND, class T>
+__device__ __forceinline__ int at(const arr<T> &f, int x, int y, int z) {
+  if (ND == 1) return x;
+  if (ND == 2) return x * f.s0 + y;
+  return x * f.s0 + y * f.s1 + z;
+}
+template <int ND, class T>
+__device__ __forceinline__ int at(const arr<T> &f, const int *c) { return at<ND>(f, c[0], c[1], c[2]); }
+
+// where coordinate q of axis d, at most 2 outside, takes a scalar from
+template <class T>
+__device__ __forceinline__ int src(const args<T> &A, int d, int q) {
+  const int n = A.n[d];
+  if (q >= 0 && q < n) return q;
+  const int side = q < 0 ? 0 : 1, kind = A.bc[d][side];
+  if (kind == MPDX_BC_CYCLIC) return side ? q - (n - 1) : q + (n - 1);
+  if (kind == MPDX_BC_OPEN) return side ? n - 1 : 0;
+  return side ? 2 * (n - 1) - q : -q;  // rigid: mirror about the wall point
+}
+// the same for a transverse axis of a velocity component; false where its fill is zero
+template <class T>
+__device__ __forceinline__ bool vsrc(const args<T> &A, int d, int &q) {
+  if (q >= 0 && q < A.n[d]) return true;
+  if (A.bc[d][q < 0 ? 0 : 1] == MPDX_BC_OPEN) return false;
+  q = src(A, d, q);
+  return true;
+}
+
+// point of the interior owned by this thread (false: none)
+template <int ND, class T>
+__device__ __forceinline__ bool own(const args<T> &A, int c[3]) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= A.plane) return false;
+  if (ND == 1) { c[0] = p; c[1] = c[2] = 0; }
+  if (ND == 2) { c[0] = int(unsigned(p) / unsigned(A.n[1])); c[1] = p - c[0] * A.n[1]; c[2] = 0; }
+  if (ND == 3) { c[0] = blockIdx.y; c[1] = int(unsigned(p) / unsigned(A.n[2])); c[2] = p - c[1] * A.n[2]; }
+  return true;
+}
+// index into the list that the blocks from nb on work through
+__device__ __forceinline__ long long list_index(int nb) {
+  return ((long long)(blockIdx.x - nb) * gridDim.y + blockIdx.y) * blockDim.x + threadIdx.x;
+}
+// entry q of the list of faces of the grid: axis d, position in the plane across it
+// (its two axes in order); false beyond the list.  Axis after axis, n_sides entries
+// per position.
+template <int ND, class T>
+__device__ __forceinline__ bool face_entry(const args<T> &A, long long q, int n_sides, int &d, int &side, int c[3]) {
+#pragma unroll
+  for (d = 0; d < ND; ++d) {
+    const int a = d == 0 ? 1 : 0, b = d == 2 ? 1 : 2;  // the other axes
+    const int na = ND > 1 ? A.n[a] : 1, nb = ND > 2 ? A.n[b] : 1;
+    const long long m = (long long)na * nb;
+    if (q < m * n_sides) {
+      side = q >= m ? 1 : 0;
+      const int w = int(q - (side ? m : 0));
+      c[0] = c[1] = c[2] = 0;
+      if (ND > 1) c[a] = w / nb;
+      if (ND > 2) c[b] = w - c[a] * nb;
+      return true;
+    }
+    q -= m * n_sides;
+  }
+  return false;
+}
+
+// ---- donor cell ----
+// fluxes through the two faces of a cell along axis d under the rigid rule for
+// fluxes (xchng_flux): F(-1) = -F(0), F(n-1) = -F(n-2)
+template <class T, class F>
+__device__ __forceinline__ T net(const args<T> &A, int d, int c, F &&f) {  // -F(+1/2) + F(-1/2)
+  T hi = f(0), lo = f(-1);
+  if (c == 0 && A.bc[d][0] == MPDX_BC_RIGID) lo = -hi;
+  else if (c == A.n[d] - 1 && A.bc[d][1] == MPDX_BC_RIGID) hi = -lo;
+  return -hi + lo;
+}
+template <int ND, class T>
+__device__ __forceinline__ T donor(T p, const T *nt) {
+  if (ND == 1) return p + nt[0];
+  if (ND == 2) return p + (nt[0] + nt[1]);
+  return p + (nt[0] + nt[1] + nt[2]);
+}
+
+template <int ND, class T>
+__global__ void __launch_bounds__(256) k_upwind(const __grid_constant__ args<T> A) {
+  const eqn<T> &E = A.e[blockIdx.z];
+  int c[3];
+  if (!own<ND>(A, c)) return;
+  const T *p = E.in.o;
+  const int o = at<ND>(E.in, c);
+  const T p0 = p[o];
+  T nt[3];
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    int a[3] = {c[0], c[1], c[2]}, b[3] = {c[0], c[1], c[2]};
+    a[d] = src(A, d, c[d] + 1);
+    b[d] = src(A, d, c[d] - 1);
+    const T pp = p[at<ND>(E.in, a)], pm = p[at<ND>(E.in, b)];
+    const T *g = E.unco[d].o;
+    const int og = at<ND>(E.unco[d], c), sg = d == ND - 1 ? 1 : (d == 0 ? E.unco[d].s0 : E.unco[d].s1);
+    const T g1 = g[og], g0 = g[og - sg];
+    nt[d] = net(A, d, c[d], [&](int f) { return f == 0 ? flux(g1, p0, pp) : flux(g0, pm, p0); });
+  }
+  E.out.o[o] = donor<ND>(p0, nt);
+}
+
+// ---- antidiffusive velocity ----
+template <class T> __device__ __forceinline__ T frac(T nom, T den) { return nom / (den + lim<T>::tiny()); }
+template <bool IGA, class T> __device__ __forceinline__ T nd4(T a, T b, T c, T d) {
+  if (IGA) return (a + b - c - d) / T(4);
+  return frac(a + b - c - d, a + b + c + d);
+}
+template <bool IGA, class T> __device__ __forceinline__ T nd2(T a, T b, T c, T d) {
+  if (IGA) return T(2) * (a - b - c + d) / T(4);
+  return T(2) * frac(a - b - c + d, a + b + c + d);
+}
+template <class T> __device__ __forceinline__ T cxx(T C) { return div6(T(3) * C * fabs(C) - T(2) * (C * C * C) - C); }
+template <class T> __device__ __forceinline__ T cxy(T C, T g) { return (fabs(C) - T(2) * (C * C)) * g / T(2); }
+
+// component D at the face c[D] + 1/2, from psi at x[d][m + 1] for coordinate c[d] + m
+// (m = -1 .. 2 along D, -1 .. 1 across), its own advector component at c, and the
+// transverse components at coordinate v[m] along D for m = 0, 1 (z[m]: they are zero)
+template <int ND, int D, bool IGA, bool TOT, class T>
+__device__ __forceinline__ T antidiff(const eqn<T> &E, const int c[3], const int (&x)[3][4], const int (&v)[2], const bool (&z)[2]) {
+  constexpr int D1 = (D + 1) % ND, D2 = (D + 2) % ND;
+  auto ps = [&](int a, int b, int e) {  // offsets along D, D1, D2
+    int w[3] = {0, 0, 0};
+    w[D] = x[D][a + 1];
+    if (ND > 1) w[D1] = x[D1][b + 1];
+    if (ND > 2) w[D2] = x[D2][e + 1];
+    return E.in.o[at<ND>(E.in, w)];
+  };
+  auto bar = [&](auto qq) {  // average of component q over the four faces around
+    constexpr int q = decltype(qq)::value;
+    auto gq = [&](int a, int b) {
+      if (z[a]) return T(0);
+      int w[3] = {c[0], c[1], c[2]};
+      w[D] = v[a];
+      w[q] = c[q] + b;
+      return E.unco[q].o[at<ND>(E.unco[q], w)];
+    };
+    return (gq(1, 0) + gq(0, 0) + gq(1, -1) + gq(0, -1)) / T(4);
+  };
+  const T C = E.unco[D].o[at<ND>(E.unco[D], c)];
+  const T p1 = ps(1, 0, 0), p0 = ps(0, 0, 0);
+  T ndx;
+  if (IGA) ndx = ND == 3 ? p1 - p0 : T(2) * (p1 - p0) / T(2);
+  else ndx = T(2) * frac(p1 - p0, p1 + p0);
+  T r = fabs(C) / T(2) * (T(1) - fabs(C)) * ndx;
+  T xx = T(0);
+  if (TOT) xx = nd2<IGA>(ps(2, 0, 0), p1, p0, ps(-1, 0, 0));
+  if constexpr (ND == 1) {
+    if (TOT) r = r + xx * cxx(C);
+  } else if constexpr (ND == 2) {
+    const T gc1 = bar(ic<D1>{});
+    const T a = ps(1, 1, 0), b = ps(0, 1, 0), e = ps(1, -1, 0), f = ps(0, -1, 0);
+    r = r - C * gc1 / T(2) * nd4<IGA>(a, b, e, f);
+    if (TOT) r = r + (xx * cxx(C) + nd2<IGA>(a, b, e, f) * cxy(C, gc1));
+  } else {
+    const T gc1 = bar(ic<D1>{}), gc2 = bar(ic<D2>{});
+    const T a = ps(1, 1, 0), b = ps(0, 1, 0), e = ps(1, -1, 0), f = ps(0, -1, 0);
+    const T a2 = ps(1, 0, 1), b2 = ps(0, 0, 1), e2 = ps(1, 0, -1), f2 = ps(0, 0, -1);
+    r = r - C / T(2) * (gc1 * nd4<IGA>(a, b, e, f) + gc2 * nd4<IGA>(a2, b2, e2, f2));
+    if (TOT) {
+      const T q0 = ps(1, 1, 1), q1 = ps(1, -1, -1), q2 = ps(1, 1, -1), q3 = ps(1, -1, 1);
+      const T q4 = ps(0, 1, 1), q5 = ps(0, -1, -1), q6 = ps(0, 1, -1), q7 = ps(0, -1, 1);
+      const T nom = q0 + q1 - q2 - q3 + q4 + q5 - q6 - q7;
+      const T yz = IGA ? nom / T(8) : frac(nom, q0 + q1 + q2 + q3 + q4 + q5 + q6 + q7);
+      r = r + (xx * cxx(C) + nd2<IGA>(a, b, e, f) * cxy(C, gc1) + nd2<IGA>(a2, b2, e2, f2) * cxy(C, gc2)
+               + yz * div3(T(-2) * C * gc1 * gc2));
+    }
+  }
+  return r;
+}
+
+// Component D at c (c[D] = -1 .. n-1), stored.  HALO: the advector being corrected has
+// its halo in memory (the solver's own); otherwise it is the velocity of the previous
+// pass, read by the rule of its fill.  With fct the faces -1 and n-1 get what the
+// along-axis fill leaves there: a cyclic axis the copies of faces n-2 and 0 (evaluated
+// there), an open neighbouring side zero on the edges of the domain.  IN: the whole
+// stencil lies in the interior.
+template <int ND, int D, bool IGA, bool TOT, bool HALO, bool IN, class T>
+__device__ __forceinline__ void antidiff_face(const args<T> &A, const eqn<T> &E, const int c[3], bool fct) {
+  int cc[3] = {c[0], c[1], c[2]}, x[3][4], v[2];
+  bool zero = false, z[2] = {false, false};
+  if (!IN && fct) {
+    const int n = A.n[D];
+    if (A.bc[D][0] == MPDX_BC_CYCLIC) {
+      if (c[D] == -1) cc[D] = n - 2;
+      else if (c[D] == n - 1) cc[D] = 0;
+    } else if (c[D] == -1 || c[D] == n - 1) {
+#pragma unroll
+      for (int d = 0; d < D; ++d)
+        zero = zero || (c[d] == 0 && A.bc[d][0] == MPDX_BC_OPEN) || (c[d] == A.n[d] - 1 && A.bc[d][1] == MPDX_BC_OPEN);
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int m = -1; m <= 2; ++m) x[d][m + 1] = d >= ND || (m == 2 && !(TOT && d == D)) ? 0 : (IN ? cc[d] + m : src(A, d, cc[d] + m));
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    v[m] = cc[D] + m;
+    if (!HALO && !IN) z[m] = !vsrc(A, D, v[m]);
+  }
+  const T r = antidiff<ND, D, IGA, TOT>(E, cc, x, v, z);
+  E.corr[D].o[at<ND>(E.corr[D], c)] = zero ? T(0) : r;
+}
+
+template <int ND, bool IGA, bool TOT, bool HALO, class T>
+__global__ void __launch_bounds__(256) k_antidiff(const __grid_constant__ args<T> A, int nb, bool fct) {
+  const eqn<T> &E = A.e[blockIdx.z];
+  int c[3];
+  if (int(blockIdx.x) < nb) {
+    if (!own<ND>(A, c)) return;
+    bool in = true;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) in = in && c[d] >= 1 && c[d] <= A.n[d] - 3;
+    if (__all_sync(__activemask(), in)) {
+      antidiff_face<ND, 0, IGA, TOT, HALO, true>(A, E, c, fct);
+      if constexpr (ND > 1) antidiff_face<ND, 1, IGA, TOT, HALO, true>(A, E, c, fct);
+      if constexpr (ND > 2) antidiff_face<ND, 2, IGA, TOT, HALO, true>(A, E, c, fct);
+    } else {
+      antidiff_face<ND, 0, IGA, TOT, HALO, false>(A, E, c, fct);
+      if constexpr (ND > 1) antidiff_face<ND, 1, IGA, TOT, HALO, false>(A, E, c, fct);
+      if constexpr (ND > 2) antidiff_face<ND, 2, IGA, TOT, HALO, false>(A, E, c, fct);
+    }
+    return;
+  }
+  int d, side;
+  if (!face_entry<ND>(A, list_index(nb), 1, d, side, c)) return;
+  c[d] = -1;
+  if (d == 0) antidiff_face<ND, 0, IGA, TOT, HALO, false>(A, E, c, fct);
+  if constexpr (ND > 1) if (d == 1) antidiff_face<ND, 1, IGA, TOT, HALO, false>(A, E, c, fct);
+  if constexpr (ND > 2) if (d == 2) antidiff_face<ND, 2, IGA, TOT, HALO, false>(A, E, c, fct);
+}
+
+// ---- FCT limiters ----
+// antidiffusive velocity d one face beyond the stored ones (c[d] = -2 or n), the other
+// coordinates interior: the along-axis fill with ad (bcond/{cyclic,open,rigid}_*.hpp)
+template <int ND, int D, class T>
+__device__ __forceinline__ T beyond(const args<T> &A, const eqn<T> &E, int side, const int c[3]) {
+  const int n = A.n[D], kind = A.bc[D][side];
+  int w[3] = {c[0], c[1], c[2]};
+  const arr<T> &f = E.corr[D];
+  if (kind == MPDX_BC_CYCLIC) { w[D] = side ? 1 : n - 3; return f.o[at<ND>(f, w)]; }
+  if (kind == MPDX_BC_RIGID) { w[D] = side ? n - 2 : 1; return -f.o[at<ND>(f, w)]; }
+  if (ND == 1) { w[D] = side ? n - 3 : 0; return f.o[at<ND>(f, w)]; }  // open_1d.hpp with a halo of 2
+  const int e = side ? n - 1 : 0;
+  w[D] = side ? e - 1 : e;
+  T r = f.o[at<ND>(f, w)];
+  w[D] = e;
+  // zero divergence in the edge cell; the components after D are zero on the edges of
+  // the domain at this point of the fill's order
+  auto across = [&](auto qq) {
+    constexpr int q = decltype(qq)::value;
+    const arr<T> &g = E.corr[q];
+    int lo[3] = {w[0], w[1], w[2]};
+    lo[q] = w[q] - 1;
+    const T a = q > D && lo[q] == -1 ? T(0) : g.o[at<ND>(g, lo)];
+    const T b = q > D && w[q] == A.n[q] - 1 ? T(0) : g.o[at<ND>(g, w)];
+    return a - b;
+  };
+  if constexpr (ND > 1) r = side ? r + across(ic<(D + 1) % ND>{}) : r - across(ic<(D + 1) % ND>{});
+  if constexpr (ND > 2) r = side ? r + across(ic<(D + 2) % ND>{}) : r - across(ic<(D + 2) % ND>{});
+  return r;
+}
+
+// MODE 0: psi_min / psi_max from psin; 1: the same, and stored for the next pass; 2: as
+// stored.  c: a cell of the interior, or one just outside along axis `out` (-1: none).
+template <int ND, bool IGA, int MODE, bool IN, class T>
+__device__ __forceinline__ void beta_cell(const args<T> &A, const eqn<T> &E, const int c[3], int out) {
+  int x[3][3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) x[d][m] = d >= ND ? 0 : (IN ? c[d] + m - 1 : src(A, d, c[d] + m - 1));
+  auto off = [&](int d, int m) {  // one step along d
+    int w[3] = {x[0][1], x[1][1], x[2][1]};
+    if (d < ND) w[d] = x[d][m + 1];
+    return at<ND>(E.in, w);
+  };
+  const int o0 = off(3, 0);
+  int oh[3], ol[3];
+  T ph[3], pl[3];
+  const T p0 = E.in.o[o0];
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    oh[d] = off(d, 1); ol[d] = off(d, -1);
+    ph[d] = E.in.o[oh[d]]; pl[d] = E.in.o[ol[d]];
+  }
+  // velocities through the upper and lower face along each axis
+  T hi[3], lo[3];
+  auto faces = [&](auto dd) {
+    constexpr int d = decltype(dd)::value;
+    const arr<T> &f = E.corr[d];
+    int w[3] = {c[0], c[1], c[2]};
+    bool zero = false;
+    if (!IN && out >= 0 && out != d) zero = !vsrc(A, out, w[out]);
+    const int ow = at<ND>(f, w), sd = d == ND - 1 ? 1 : (d == 0 ? f.s0 : f.s1);
+    if (!IN && out == d) {
+      const int side = c[d] < 0 ? 0 : 1;
+      hi[d] = side ? beyond<ND, d>(A, E, 1, c) : f.o[ow];
+      lo[d] = side ? f.o[ow - sd] : beyond<ND, d>(A, E, 0, c);
+    } else {
+      hi[d] = zero ? T(0) : f.o[ow];
+      lo[d] = zero ? T(0) : f.o[ow - sd];
+    }
+    if (!IGA) { hi[d] = flux(hi[d], p0, ph[d]); lo[d] = flux(lo[d], pl[d], p0); }
+  };
+  faces(ic<0>{});
+  if constexpr (ND > 1) faces(ic<1>{});
+  if constexpr (ND > 2) faces(ic<2>{});
+  const int oc = at<ND>(E.bu, c);
+  T mn, mx;
+  if (MODE == 2) {
+    mn = E.mn.o[oc]; mx = E.mx.o[oc];
+  } else {
+    const T *q = E.psin.o;
+    const T q0 = q[o0];
+    if (ND == 1) {
+      const T l = q[ol[0]], h = q[oh[0]];
+      mn = dmin(dmin(l, q0), h);
+      mx = dmax(dmax(l, q0), h);
+    } else if (ND == 2) {
+      const T xl = q[ol[0]], xh = q[oh[0]], yl = q[ol[1]], yh = q[oh[1]];
+      mn = dmin(dmin(dmin(dmin(yh, xl), q0), xh), yl);
+      mx = dmax(dmax(dmax(dmax(yh, xl), q0), xh), yl);
+    } else {
+      const T xl = q[ol[0]], xh = q[oh[0]], yl = q[ol[1]], yh = q[oh[1]], zl = q[ol[2]], zh = q[oh[2]];
+      mn = dmin(dmin(dmin(dmin(dmin(dmin(q0, xh), xl), yh), yl), zh), zl);
+      mx = dmax(dmax(dmax(dmax(dmax(dmax(q0, xh), xl), yh), yl), zh), zl);
+    }
+    if (MODE == 1) { E.mn.o[oc] = mn; E.mx.o[oc] = mx; }
+  }
+  T du, dd;
+  if (ND == 1) {
+    mx = dmax(mx, dmax(pl[0], dmax(p0, ph[0])));
+    mn = dmin(mn, dmin(pl[0], dmin(p0, ph[0])));
+    du = pos(lo[0]) - neg(hi[0]);
+    dd = pos(hi[0]) - neg(lo[0]);
+  } else if (ND == 2) {
+    mx = dmax(mx, dmax(ph[1], dmax(pl[0], dmax(p0, dmax(ph[0], pl[1])))));
+    mn = dmin(mn, dmin(ph[1], dmin(pl[0], dmin(p0, dmin(ph[0], pl[1])))));
+    du = (pos(lo[0]) - neg(hi[0])) + (pos(lo[1]) - neg(hi[1]));
+    dd = (pos(hi[0]) - neg(lo[0])) + (pos(hi[1]) - neg(lo[1]));
+  } else {
+    mx = dmax(mx, dmax(p0, dmax(ph[0], dmax(pl[0], dmax(ph[1], dmax(pl[1], dmax(ph[2], pl[2])))))));
+    mn = dmin(mn, dmin(ph[1], dmin(pl[0], dmin(p0, dmin(ph[0], dmin(ph[2], dmin(pl[2], pl[1])))))));
+    du = (pos(lo[0]) - neg(hi[0])) + (pos(lo[1]) - neg(hi[1])) + (pos(lo[2]) - neg(hi[2]));
+    dd = (pos(hi[0]) - neg(lo[0])) + (pos(hi[1]) - neg(lo[1])) + (pos(hi[2]) - neg(lo[2]));
+  }
+  E.bu.o[oc] = (mx - p0) / (du + lim<T>::eps());
+  E.bd.o[oc] = (p0 - mn) / (dd + lim<T>::eps());
+}
+
+template <int ND, bool IGA, int MODE, class T>
+__global__ void __launch_bounds__(256) k_betas(const __grid_constant__ args<T> A, int nb) {
+  const eqn<T> &E = A.e[blockIdx.z];
+  int c[3];
+  if (int(blockIdx.x) < nb) {
+    if (!own<ND>(A, c)) return;
+    bool in = true;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) in = in && c[d] >= 1 && c[d] <= A.n[d] - 2;
+    if (__all_sync(__activemask(), in)) beta_cell<ND, IGA, MODE, true>(A, E, c, -1);
+    else beta_cell<ND, IGA, MODE, false>(A, E, c, -1);
+    return;
+  }
+  int d, side;
+  if (!face_entry<ND>(A, list_index(nb), 2, d, side, c)) return;
+  c[d] = side ? A.n[d] : -1;
+  beta_cell<ND, IGA, MODE, false>(A, E, c, d);
+}
+
+// ---- corrective donor-cell pass ----
+template <int ND, bool IGA, bool FCT, class T>
+__global__ void __launch_bounds__(256) k_correct(const __grid_constant__ args<T> A) {
+  const eqn<T> &E = A.e[blockIdx.z];
+  int c[3];
+  if (!own<ND>(A, c)) return;
+  const int o = at<ND>(E.in, c);
+  const T p0 = E.in.o[o];
+  T bu0 = T(0), bd0 = T(0);
+  if (FCT) { bu0 = E.bu.o[o]; bd0 = E.bd.o[o]; }
+  auto limited = [](T C, T bul, T bdl, T bur, T bdr) {  // GC_mono (l: cell below the face, r: above)
+    return C * (C > T(0) ? dmin(T(1), dmin(bdl, bur)) : dmin(T(1), dmin(bul, bdr)));
+  };
+  T nt[3];
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    const arr<T> &f = E.corr[d];
+    const int of = at<ND>(f, c), sf = d == ND - 1 ? 1 : (d == 0 ? f.s0 : f.s1);
+    const int so = d == ND - 1 ? 1 : (d == 0 ? E.bu.s0 : E.bu.s1);
+    T ch = f.o[of], cl = f.o[of - sf];
+    if (FCT) {
+      ch = limited(ch, bu0, bd0, E.bu.o[o + so], E.bd.o[o + so]);
+      cl = limited(cl, E.bu.o[o - so], E.bd.o[o - so], bu0, bd0);
+    }
+    T pp = T(0), pm = T(0);
+    if (!IGA) {
+      int a[3] = {c[0], c[1], c[2]}, b[3] = {c[0], c[1], c[2]};
+      a[d] = src(A, d, c[d] + 1);
+      b[d] = src(A, d, c[d] - 1);
+      pp = E.in.o[at<ND>(E.in, a)];
+      pm = E.in.o[at<ND>(E.in, b)];
+    }
+    nt[d] = net(A, d, c[d], [&](int w) { return IGA ? (w == 0 ? ch : cl) : (w == 0 ? flux(ch, p0, pp) : flux(cl, pm, p0)); });
+  }
+  E.out.o[o] = donor<ND>(p0, nt);
+}
+
+// ---- host ----
+template <class T>
+arr<T> view(const field<T> &f) {
+  return {f.v.o, int(f.v.s0), int(f.v.s1)};
+}
+
+template <class T, int ND>
+void step_nd(mpdata_state<T> &st, stage_engine<T> &eng, int e0, int ne, int passes) {
+  args<T> A;
+  for (int d = 0; d < 3; ++d) {
+    A.n[d] = st.n[d];
+    A.bc[d][0] = st.bcs[d][0];
+    A.bc[d][1] = st.bcs[d][1];
+  }
+  A.plane = int(ND == 3 ? (long long)st.n[1] * st.n[2] : (ND == 2 ? (long long)st.n[0] * st.n[1] : st.n[0]));
+  const bool fct = st.opts & o_fct, iga = st.opts & o_iga, tot = st.opts & o_tot;
+  const int bs = 256, nb = int(ceil_div(A.plane, bs)), ny = ND == 3 ? st.n[0] : 1;
+  const dim3 grid(nb, ny, ne);
+  long long faces = 0;  // positions of one face per axis
+  for (int d = 0; d < ND; ++d) faces += st.cells() / st.n[d];
+  auto with_list = [&](long long entries) { return dim3(nb + ceil_div(entries, (long long)bs * ny), ny, ne); };
+  cudaStream_t s = st.stream;
+  for (int it = 0; it < passes; ++it) {
+    for (int q = 0; q < ne; ++q) {
+      eqn<T> &E = A.e[q];
+      const int e = e0 + q, tl = st.tl[e];
+      typename stage_engine<T>::work *w = q > 0 ? &eng.more[q - 1] : nullptr;
+      field<T> *t0 = w ? w->tmp0 : st.tmp0, *t1 = w ? w->tmp1 : st.tmp1;
+      E.in = view(st.psi[e][tl ^ (it & 1)]);
+      E.out = view(st.psi[e][tl ^ (it & 1) ^ 1]);
+      E.psin = view(st.psi[e][tl]);
+      for (int d = 0; d < 3; ++d) {
+        const int dd = d < ND ? d : 0;
+        E.corr[d] = view(it == 2 ? t1[dd] : t0[dd]);
+        E.unco[d] = view(it < 2 ? st.GC[dd] : t0[dd]);
+      }
+      if (fct) {
+        E.bu = view(w ? w->beta_up : st.beta_up);
+        E.bd = view(w ? w->beta_dn : st.beta_dn);
+        E.mn = view(w ? w->psi_min : st.psi_min);
+        E.mx = view(w ? w->psi_max : st.psi_max);
+      }
+    }
+    if (it == 0) {
+      k_upwind<ND><<<grid, bs, 0, s>>>(A);
+      MPDX_LAUNCH_CHECK();
+      continue;
+    }
+    const dim3 ga = with_list(faces), gb = with_list(2 * faces);
+    auto anti = [&](auto ig, auto to) {
+      constexpr bool IG = decltype(ig)::value, TO = decltype(to)::value;
+      if (it == 1) k_antidiff<ND, IG, TO, true><<<ga, bs, 0, s>>>(A, nb, fct);
+      else k_antidiff<ND, IG, TO, false><<<ga, bs, 0, s>>>(A, nb, fct);
+    };
+    auto rest = [&](auto ig) {
+      constexpr bool IG = decltype(ig)::value;
+      if (fct) {
+        if (it == 2) k_betas<ND, IG, 2><<<gb, bs, 0, s>>>(A, nb);
+        else if (passes > 2) k_betas<ND, IG, 1><<<gb, bs, 0, s>>>(A, nb);
+        else k_betas<ND, IG, 0><<<gb, bs, 0, s>>>(A, nb);
+        MPDX_LAUNCH_CHECK();
+        k_correct<ND, IG, true><<<grid, bs, 0, s>>>(A);
+      } else {
+        k_correct<ND, IG, false><<<grid, bs, 0, s>>>(A);
+      }
+    };
+    if (iga && tot) anti(std::true_type{}, std::true_type{});
+    else if (iga) anti(std::true_type{}, std::false_type{});
+    else if (tot) anti(std::false_type{}, std::true_type{});
+    else anti(std::false_type{}, std::false_type{});
+    MPDX_LAUNCH_CHECK();
+    if (iga) rest(std::true_type{});
+    else rest(std::false_type{});
+    MPDX_LAUNCH_CHECK();
+  }
+  if (passes & 1)
+    for (int q = 0; q < ne; ++q) st.tl[e0 + q] ^= 1;
+}
+
+}  // namespace sg
+
+template <class T>
+bool stage_engine<T>::covers(const mpdata_state<T> &st) {
+  if (st.opts & ~(o_fct | o_iga | o_tot)) return false;
+  if (st.n_iters < 1 || st.n_iters > 3) return false;
+  bool rigid = false;
+  for (int d = 0; d < st.nd; ++d) {
+    if (st.n[d] < 2 * st.H + 1) return false;
+    for (int q = 0; q < 2; ++q) rigid = rigid || st.bcs[d][q] == MPDX_BC_RIGID;
+    if ((st.bcs[d][0] == MPDX_BC_CYCLIC) != (st.bcs[d][1] == MPDX_BC_CYCLIC)) return false;
+  }
+  // the reference then rewrites the velocity that the third pass corrects (xchng_flux
+  // on the fluxes of the infinite gauge, which are that velocity)
+  if (st.n_iters == 3 && (st.opts & o_iga) && !(st.opts & o_fct) && rigid) return false;
+  if (st.nd == 3 && st.n[0] > 65535) return false;
+  // 32-bit offsets
+  size_t most = st.psi[0][0].bytes;
+  for (int d = 0; d < st.nd; ++d) most = std::max(most, st.GC[d].bytes);
+  return most / sizeof(T) < (size_t(1) << 31) - 65536;
+}
+
+// One launch takes up to kStageEqns equations of a small grid (their work arrays
+// together stay in cache and the launches count), one of a large grid.
+constexpr long long kStageBatchCells = 1 << 18;
+
+template <class T>
+void stage_engine<T>::step(mpdata_state<T> &st, bool upwind_only) {
+  const int passes = upwind_only ? 1 : st.n_iters;
+  const int most = st.cells() <= kStageBatchCells ? kStageEqns : 1;
+  for (int e0 = 0; e0 < st.n_eqns; e0 += most) {
+    const int ne = std::min(most, st.n_eqns - e0);
+    while (passes > 1 && int(more.size()) < ne - 1) {
+      more.emplace_back();
+      auto &w = more.back();
+      st.alloc_vctr(w.tmp0);
+      if (st.n_iters > 2) st.alloc_vctr(w.tmp1);
+      if (st.opts & o_fct)
+        for (field<T> *f : {&w.beta_up, &w.beta_dn, &w.psi_min, &w.psi_max}) st.alloc_sclr(*f);
+    }
+    if (int(more.size()) < ne - 1) more.resize(ne - 1);
+    if (st.nd == 1) sg::step_nd<T, 1>(st, *this, e0, ne, passes);
+    else if (st.nd == 2) sg::step_nd<T, 2>(st, *this, e0, ne, passes);
+    else sg::step_nd<T, 3>(st, *this, e0, ne, passes);
+  }
+}
+
+}  // namespace mpdx
