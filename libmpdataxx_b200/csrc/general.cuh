@@ -40,8 +40,9 @@ struct general {
   void fill_flux(int d, int side, field<T> *AV, rng rb, rng rc);
   bool any_rigid() const;
 
- private:
   stage_engine<T> stages;  // the common options in a few launches per step
+
+ private:
   int cur_e = 0;  // equation whose advop is running (the divergence form reads its other time level)
   field<T> *GC_unco(int iter);
   field<T> *GC_corr(int iter);

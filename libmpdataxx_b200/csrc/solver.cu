@@ -253,6 +253,12 @@ struct mpdata_solver : solver_base {
   void advance(long long nt) override {
     if (nt <= 0) return;
     if (st.timestep == 0) gen.ante_loop(scratch);
+    if (path != MPDX_PATH_GENERAL && stage_engine<T>::line_covers(st) &&
+        (st.bcs[0][0] != MPDX_BC_CYCLIC || fus.seams_consistent(st, scratch))) {
+      gen.stages.line(st, nt);
+      last_path = MPDX_PATH_FUSED;
+      return;
+    }
     if (path != MPDX_PATH_GENERAL && gen.block1d_ok()) {
       gen.block1d(nt);
       st.timestep += nt;

@@ -22,6 +22,10 @@ struct stage_engine {
   static bool covers(const mpdata_state<T> &st);
   // advances every equation by one step; `upwind_only`: the first pass alone
   void step(mpdata_state<T> &st, bool upwind_only);
+  // one-dimensional problems with both ends open, or cyclic with consistent seams:
+  // nt steps, several per launch (advances st.timestep)
+  static bool line_covers(const mpdata_state<T> &st);
+  void line(mpdata_state<T> &st, long long nt);
 };
 
 extern template struct stage_engine<float>;

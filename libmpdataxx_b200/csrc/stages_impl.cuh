@@ -486,6 +486,181 @@ __global__ void __launch_bounds__(256) k_correct(const __grid_constant__ args<T>
   E.out.o[o] = donor<ND>(p0, nt);
 }
 
+// ---- one-dimensional problems: several steps per launch in registers ----
+// A warp holds 128 consecutive points, 4 per lane, and takes `steps` steps of its
+// segment alone; neighbours come by shuffles.  Every step spoils at most `radius`
+// points at each end of the segment, so the outermost steps * radius points are halo:
+// computed, not written, and no warp waits for another.  A cyclic axis whose point
+// n-1 repeats point 0 is unrolled with period n-1; outside an open axis every stage
+// takes the edge values that its halo fill would give it.  Arithmetic of the stages
+// above.  Bound by the latency of one step (divisions and shuffles in sequence) and,
+// with many segments, by issue.
+constexpr int kLinePoints = 128;
+// points that one step spoils: psi1 1, then per corrective pass the donor-cell sum 1,
+// the limiter 1 and a third-order term 1
+__host__ __device__ constexpr int line_radius(int passes, bool fct, bool tot) {
+  return 1 + (passes - 1) * (1 + (fct ? 1 : 0) + (tot ? 1 : 0));
+}
+
+template <class T>
+struct line_args {
+  const T *in[kStageEqns];
+  T *out[kStageEqns];
+  const T *gc;  // faces -hv .. n-2+hv
+  int n, steps, halo, hv;
+  bool cyclic;
+  long long t0;
+  int uff;
+};
+
+template <class T>
+struct q4 {
+  T v[4];
+  __device__ __forceinline__ T operator[](int e) const { return v[e]; }
+  __device__ __forceinline__ T &operator[](int e) { return v[e]; }
+};
+template <class T> __device__ __forceinline__ q4<T> left(const q4<T> &a) {  // values one point below
+  return {{__shfl_up_sync(0xffffffffu, a.v[3], 1), a.v[0], a.v[1], a.v[2]}};
+}
+template <class T> __device__ __forceinline__ q4<T> right(const q4<T> &a) {
+  return {{a.v[1], a.v[2], a.v[3], __shfl_down_sync(0xffffffffu, a.v[0], 1)}};
+}
+#define MPDX_EACH for (int e = 0; e < 4; ++e)
+
+template <int NI, bool FCT, bool IGA, bool TOT, class T>
+__global__ void __launch_bounds__(128) k_line(const line_args<T> A) {
+  const int lane = threadIdx.x & 31, seg = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int useful = kLinePoints - 2 * A.halo, n = A.n, P = A.cyclic ? n - 1 : n;
+  const int x0 = seg * useful;
+  if (x0 >= P) return;  // whole warps
+  const int xs = x0 - A.halo;  // first point of the segment
+  const T *const in = A.in[blockIdx.y];
+  T *const out = A.out[blockIdx.y];
+  int x[4];
+  q4<T> p, C0;
+#pragma unroll
+  MPDX_EACH {
+    x[e] = xs + 4 * lane + e;
+    int q = x[e];
+    if (A.cyclic) { q %= P; q += q < 0 ? P : 0; }
+    p[e] = in[A.cyclic ? q : min(max(q, 0), n - 1)];
+    C0[e] = A.gc[A.cyclic ? q : min(max(q, -A.hv), n - 2 + A.hv)];
+  }
+  // whether the segment reaches outside an open axis
+  const bool edge = !A.cyclic && (xs < 0 || xs + kLinePoints > n);
+  auto pick = [&](const q4<T> &a, int q) {  // value at point q of the segment
+    const int w = q - xs;
+    const T u = (w & 3) == 0 ? a[0] : ((w & 3) == 1 ? a[1] : ((w & 3) == 2 ? a[2] : a[3]));
+    return __shfl_sync(0xffffffffu, u, (w >> 2) & 31);
+  };
+  auto fill = [&](q4<T> &a) {  // open scalar fill
+    if (!edge) return;
+    const T l = pick(a, 0), r = pick(a, n - 1);
+#pragma unroll
+    MPDX_EACH {
+      if (x[e] < 0) a[e] = l;
+      if (x[e] > n - 1) a[e] = r;
+    }
+  };
+  auto fill_v = [&](q4<T> &a) {  // open along-axis fill of an antidiffusive velocity (open_1d.hpp)
+    if (!edge) return;
+    const T l = pick(a, 0), r = pick(a, n - 3);
+#pragma unroll
+    MPDX_EACH {
+      if (x[e] < -1) a[e] = l;
+      if (x[e] > n - 1) a[e] = r;
+    }
+  };
+  auto donor_cell = [&](const q4<T> &a, const q4<T> &f) {
+    const q4<T> fl = left(f);
+    q4<T> r;
+#pragma unroll
+    MPDX_EACH r[e] = a[e] + (-f[e] + fl[e]);
+    return r;
+  };
+  auto fluxes = [&](const q4<T> &c, const q4<T> &a) {
+    const q4<T> ar = right(a);
+    q4<T> f;
+#pragma unroll
+    MPDX_EACH f[e] = flux(c[e], a[e], ar[e]);
+    return f;
+  };
+  for (int s = 0; s < A.steps; ++s) {
+    q4<T> mn, mx;
+    if (FCT) {
+      fill(p);
+      const q4<T> l = left(p), r = right(p);
+#pragma unroll
+      MPDX_EACH {
+        mn[e] = dmin(dmin(l[e], p[e]), r[e]);
+        mx[e] = dmax(dmax(l[e], p[e]), r[e]);
+      }
+    } else {
+      fill(p);
+    }
+    p = donor_cell(p, fluxes(C0, p));
+    if (NI == 1 || (A.uff > 0 && (A.t0 + s) % A.uff == 0)) continue;
+    q4<T> C = C0;
+#pragma unroll
+    for (int it = 1; it < NI; ++it) {
+      fill(p);
+      const q4<T> pr = right(p), pl = left(p);
+      q4<T> prr = pr;
+      if (TOT) prr = right(pr);
+#pragma unroll
+      MPDX_EACH {
+        const T c = C[e], p1 = pr[e], p0 = p[e];
+        const T ndx = IGA ? T(2) * (p1 - p0) / T(2) : T(2) * frac(p1 - p0, p1 + p0);
+        T r = fabs(c) / T(2) * (T(1) - fabs(c)) * ndx;
+        if (TOT) r = r + nd2<IGA>(prr[e], p1, p0, pl[e]) * cxx(c);
+        C[e] = r;
+      }
+      q4<T> f;
+      if (FCT) {
+        fill_v(C);
+        f = C;
+        if (!IGA) f = fluxes(C, p);
+        const q4<T> fl = left(f);
+        q4<T> bu, bd;
+#pragma unroll
+        MPDX_EACH {
+          const T h = dmax(mx[e], dmax(pl[e], dmax(p[e], pr[e]))), l = dmin(mn[e], dmin(pl[e], dmin(p[e], pr[e])));
+          const T du = pos(fl[e]) - neg(f[e]), dd = pos(f[e]) - neg(fl[e]);
+          bu[e] = (h - p[e]) / (du + lim<T>::eps());
+          bd[e] = (p[e] - l) / (dd + lim<T>::eps());
+        }
+        const q4<T> bur = right(bu), bdr = right(bd);
+        q4<T> m;
+#pragma unroll
+        MPDX_EACH m[e] = C[e] * (C[e] > T(0) ? dmin(T(1), dmin(bd[e], bur[e])) : dmin(T(1), dmin(bu[e], bdr[e])));
+        f = m;
+        if (!IGA) f = fluxes(m, p);
+      } else {
+        f = C;
+        if (!IGA) f = fluxes(C, p);
+      }
+      p = donor_cell(p, f);
+    }
+  }
+#pragma unroll
+  MPDX_EACH {
+    if (x[e] < x0 || x[e] >= min(x0 + useful, P)) continue;
+    out[x[e]] = p[e];
+    if (A.cyclic && x[e] == 0) out[n - 1] = p[e];
+  }
+}
+#undef MPDX_EACH
+
+template <int NI, bool FCT, class T>
+void launch_line(const mpdata_state<T> &st, dim3 g, int bs, const line_args<T> &a) {
+  const bool iga = st.opts & o_iga, tot = st.opts & o_tot;
+  if (iga && tot) k_line<NI, FCT, true, true><<<g, bs, 0, st.stream>>>(a);
+  else if (iga) k_line<NI, FCT, true, false><<<g, bs, 0, st.stream>>>(a);
+  else if (tot) k_line<NI, FCT, false, true><<<g, bs, 0, st.stream>>>(a);
+  else k_line<NI, FCT, false, false><<<g, bs, 0, st.stream>>>(a);
+  MPDX_LAUNCH_CHECK();
+}
+
 // ---- host ----
 template <class T>
 arr<T> view(const field<T> &f) {
@@ -587,6 +762,58 @@ bool stage_engine<T>::covers(const mpdata_state<T> &st) {
   return most / sizeof(T) < (size_t(1) << 31) - 65536;
 }
 
+template <class T>
+bool stage_engine<T>::line_covers(const mpdata_state<T> &st) {
+  if (st.nd != 1 || !covers(st)) return false;
+  const int l = st.bcs[0][0], r = st.bcs[0][1];
+  return (l == MPDX_BC_CYCLIC && r == MPDX_BC_CYCLIC) || (l == MPDX_BC_OPEN && r == MPDX_BC_OPEN);
+}
+
+template <class T>
+void stage_engine<T>::line(mpdata_state<T> &st, long long nt) {
+  const bool fct = st.opts & o_fct, tot = st.opts & o_tot;
+  const int radius = sg::line_radius(st.n_iters, fct, tot), n = st.n[0];
+  // Steps per launch: a launch costs about as much as 10 steps, so as many as leave a
+  // quarter of a segment for results while all segments run at once (one warp per
+  // scheduler); with more segments than that the halo's work counts and half of a
+  // segment is kept.
+  const int most = sg::kLinePoints * 3 / 8 / radius, fewer = std::max(1, sg::kLinePoints / 4 / radius);
+  int dev = 0, sms = 148;
+  MPDX_CUDA(cudaGetDevice(&dev));
+  MPDX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const bool few = (long long)n * st.n_eqns <= 4LL * sms * (sg::kLinePoints - 2 * most * radius);
+  const int per = few ? most : fewer;
+  while (nt > 0) {
+    sg::line_args<T> a;
+    a.steps = int(std::min<long long>(nt, per));
+    a.halo = (a.steps * radius + 3) / 4 * 4;
+    a.n = n;
+    a.hv = st.H;
+    a.cyclic = st.bcs[0][0] == MPDX_BC_CYCLIC;
+    a.gc = st.GC[0].v.o;
+    a.t0 = st.timestep;
+    a.uff = st.upwind_filter_freq;
+    const int useful = sg::kLinePoints - 2 * a.halo, bs = few ? 32 : 128;
+    const int segs = int(ceil_div(a.cyclic ? n - 1 : n, useful));
+    for (int e0 = 0; e0 < st.n_eqns; e0 += kStageEqns) {
+      const int ne = std::min(kStageEqns, st.n_eqns - e0);
+      for (int q = 0; q < ne; ++q) {
+        a.in[q] = st.psi[e0 + q][st.tl[e0 + q]].v.o;
+        a.out[q] = st.psi[e0 + q][st.tl[e0 + q] ^ 1].v.o;
+        st.tl[e0 + q] ^= 1;
+      }
+      const dim3 g(ceil_div(segs, bs / 32), ne);
+      if (st.n_iters == 1) sg::launch_line<1, false>(st, g, bs, a);
+      else if (st.n_iters == 2 && fct) sg::launch_line<2, true>(st, g, bs, a);
+      else if (st.n_iters == 2) sg::launch_line<2, false>(st, g, bs, a);
+      else if (fct) sg::launch_line<3, true>(st, g, bs, a);
+      else sg::launch_line<3, false>(st, g, bs, a);
+    }
+    st.timestep += a.steps;
+    nt -= a.steps;
+  }
+}
+
 // One launch takes up to kStageEqns equations of a small grid (their work arrays
 // together stay in cache and the launches count), one of a large grid.
 constexpr long long kStageBatchCells = 1 << 18;
@@ -597,15 +824,15 @@ void stage_engine<T>::step(mpdata_state<T> &st, bool upwind_only) {
   const int most = st.cells() <= kStageBatchCells ? kStageEqns : 1;
   for (int e0 = 0; e0 < st.n_eqns; e0 += most) {
     const int ne = std::min(most, st.n_eqns - e0);
-    while (passes > 1 && int(more.size()) < ne - 1) {
-      more.emplace_back();
-      auto &w = more.back();
+    if (int(more.size()) < ne - 1) more.resize(ne - 1);
+    for (int q = 0; passes > 1 && q < ne - 1; ++q) {
+      auto &w = more[q];
+      if (w.tmp0[0].base) continue;
       st.alloc_vctr(w.tmp0);
       if (st.n_iters > 2) st.alloc_vctr(w.tmp1);
       if (st.opts & o_fct)
         for (field<T> *f : {&w.beta_up, &w.beta_dn, &w.psi_min, &w.psi_max}) st.alloc_sclr(*f);
     }
-    if (int(more.size()) < ne - 1) more.resize(ne - 1);
     if (st.nd == 1) sg::step_nd<T, 1>(st, *this, e0, ne, passes);
     else if (st.nd == 2) sg::step_nd<T, 2>(st, *this, e0, ne, passes);
     else sg::step_nd<T, 3>(st, *this, e0, ne, passes);
