@@ -250,6 +250,20 @@ struct mpdata_solver : solver_base {
     view(kind, idx, ex, off, f);
     xfer.get(stream, *f, dst, device, ex, off);
   }
+  // Where a step in stages (general<T>::step) beats the fused kernel on a periodic grid.
+  // us per step, fused and stages.  FP64 3D always (the fused canvas of 16 x 64 computes
+  // 1.83 points per result and is bound by FP64 issue): 24^3 168 and 25, 96^3 172 and
+  // 80, 250 x 257 x 241 1443 and 996, 400^3 5093 and 4535.  FP32 3D while the march
+  // of a chunk is mostly latency: 96^3 110 and 61, 160^3 112 and 200.  FP64 2D: three
+  // passes 128^2 134 and 34, 1024^2 200 and 112, 4096^2 1476 and 1446; two passes 512^2
+  // 43 and 26, 1024^2 44 and 47.  FP32 2D stays with the fused kernel, whose results
+  // equal the batched advance's bit for bit.
+  bool stages_faster() const {
+    if (!stage_engine<T>::covers(st)) return false;
+    const bool dbl = sizeof(T) == 8;
+    if (st.nd == 3) return dbl || (st.cells() <= 1000000 && fused3d_planes_setting(-1) == 0);
+    return dbl && st.cells() <= (st.n_iters == 3 ? 16000000 : 600000);
+  }
   void advance(long long nt) override {
     if (nt <= 0) return;
     if (st.timestep == 0) gen.ante_loop(scratch);
@@ -272,8 +286,9 @@ struct mpdata_solver : solver_base {
         throw error(MPDX_E_UNSUPPORTED, "fused path requested but the periodic seams of the fields are inconsistent");
     }
     last_path = use_fused ? MPDX_PATH_FUSED : MPDX_PATH_GENERAL;
+    const bool one_kernel = use_fused && !(path == MPDX_PATH_AUTO && stages_faster());
     for (long long t = 0; t < nt; ++t) {
-      if (use_fused) fus.step(st);
+      if (one_kernel) fus.step(st);
       else gen.step();
       ++st.timestep;
     }
