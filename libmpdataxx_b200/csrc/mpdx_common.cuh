@@ -46,6 +46,27 @@ struct error : std::runtime_error {
 
 #define MPDX_LAUNCH_CHECK() MPDX_CUDA(cudaGetLastError())
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may start
+// while the kernel before it in the stream still runs its last blocks, and calls
+// after_previous() before it touches memory (it returns when that kernel has ended and
+// its stores are visible); next_may_start() lets the kernel after it do the same.
+// Hides the launch latency and index arithmetic of chains of short kernels.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+void launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t s, A &&...a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  MPDX_CUDA(cudaLaunchKernelEx(&c, kern, P(a)...));
+}
+
 struct rng {
   int f, l;
   int n() const { return l - f + 1; }
