@@ -137,13 +137,16 @@ __device__ __forceinline__ bool face_entry(const args<T> &A, long long q, int n_
   return false;
 }
 
+// Threads per block: 128; with 256 the waits at the ends of blocks cost 2 to 9 % more
+// (1024^2 in three passes 103.5 and 95.6 us per step, 256 x 256 x 128 FP32 371 and 359).
+constexpr int kStageThreads = 128;
 // Blocks per SM that the registers are kept for: the kernels wait on L2 and DRAM, and
 // the walk's carried values would otherwise leave 8 warps per SM (k_antidiff at 150
 // registers).  250 x 257 x 241 iga|fct, us per step without and with: FP64 1240 and 996,
 // FP32 657 and 633.
 template <class T> struct blocks;
-template <> struct blocks<float> { static constexpr int upwind = 5, antidiff = 3, betas = 4, correct = 5; };
-template <> struct blocks<double> { static constexpr int upwind = 6, antidiff = 2, betas = 4, correct = 6; };
+template <> struct blocks<float> { static constexpr int upwind = 10, antidiff = 6, betas = 8, correct = 10; };
+template <> struct blocks<double> { static constexpr int upwind = 12, antidiff = 4, betas = 8, correct = 12; };
 
 // The march of the 2D and 3D kernels: a thread owns a position of the axes after the
 // first and walks `mi` planes along axis 0, so that positions, halo rules and offsets
@@ -186,7 +189,7 @@ __device__ __forceinline__ T donor(T p, const T *nt) {
 }
 
 template <int ND, class T>
-__global__ void __launch_bounds__(256, blocks<T>::upwind) k_upwind(const __grid_constant__ args<T> A, int mi) {
+__global__ void __launch_bounds__(kStageThreads, blocks<T>::upwind) k_upwind(const __grid_constant__ args<T> A, int mi) {
   next_may_start();
   const eqn<T> &E = A.e[blockIdx.z];
   if constexpr (ND == 1) {
@@ -341,7 +344,7 @@ __device__ __forceinline__ void antidiff_face(const args<T> &A, const eqn<T> &E,
 }
 
 template <int ND, bool IGA, bool TOT, bool HALO, class T>
-__global__ void __launch_bounds__(256, blocks<T>::antidiff) k_antidiff(const __grid_constant__ args<T> A, int nb, int mi, bool fct) {
+__global__ void __launch_bounds__(kStageThreads, blocks<T>::antidiff) k_antidiff(const __grid_constant__ args<T> A, int nb, int mi, bool fct) {
   next_may_start();
   const eqn<T> &E = A.e[blockIdx.z];
   if (ND == 1 || int(blockIdx.x) >= nb) {
@@ -591,7 +594,7 @@ __device__ __forceinline__ void beta_cell(const args<T> &A, const eqn<T> &E, con
 }
 
 template <int ND, bool IGA, int MODE, class T>
-__global__ void __launch_bounds__(256, blocks<T>::betas) k_betas(const __grid_constant__ args<T> A, int nb, int mi) {
+__global__ void __launch_bounds__(kStageThreads, blocks<T>::betas) k_betas(const __grid_constant__ args<T> A, int nb, int mi) {
   next_may_start();
   const eqn<T> &E = A.e[blockIdx.z];
   if (ND == 1 || int(blockIdx.x) >= nb) {
@@ -657,7 +660,7 @@ __device__ __forceinline__ T limited(T C, T bul, T bdl, T bur, T bdr) {  // GC_m
 }
 
 template <int ND, bool IGA, bool FCT, class T>
-__global__ void __launch_bounds__(256, blocks<T>::correct) k_correct(const __grid_constant__ args<T> A, int mi) {
+__global__ void __launch_bounds__(kStageThreads, blocks<T>::correct) k_correct(const __grid_constant__ args<T> A, int mi) {
   next_may_start();
   const eqn<T> &E = A.e[blockIdx.z];
   if constexpr (ND == 1) {
@@ -902,13 +905,13 @@ void launch_line(const mpdata_state<T> &st, dim3 g, int bs, const line_args<T> &
 }
 
 // ---- host ----
-// Planes that a thread walks: at most 8, at least 2, halved while fewer than 1000 blocks
-// would run.  FP64 us per step for 1, 2, 4, 8 and 16 planes: 59^3 fct 51, 42, 46, 61,
-// 91; 1024^2 fct in three passes 127, 112, 113, 119, 160; 250 x 257 x 241 iga|fct 1862,
-// 1141, 1028, 996, 1224 (the last before the register limits of `blocks`).
+// Planes that a thread walks: at most 8, halved while fewer than 1100 blocks would run.
+// FP64 us per step for 1, 2, 4 and 8 planes: 59^3 fct 36, 39, 47, 69; 97 x 89 x 65
+// iga|fct 61, 55, 54, 76; 1024^2 fct in three passes 112, 97, 96, 119;
+// 250 x 257 x 241 iga|fct 1419, 1099, 989, 976.
 inline int planes_per_thread(int n0, long long blocks) {
   int mi = 8;
-  while (mi > 2 && blocks * ceil_div(n0, mi) < 1000) mi /= 2;
+  while (mi > 1 && blocks * ceil_div(n0, mi) < 1100) mi /= 2;
   while (ceil_div(n0, mi) > 65535) mi *= 2;  // blocks along the grid's second axis
   return mi;
 }
@@ -927,7 +930,7 @@ void step_nd(mpdata_state<T> &st, stage_engine<T> &eng, int e0, int ne, int pass
     A.bc[d][1] = st.bcs[d][1];
   }
   const bool fct = st.opts & o_fct, iga = st.opts & o_iga, tot = st.opts & o_tot;
-  const int bs = 256, pos = ND == 1 ? st.n[0] : (ND == 2 ? st.n[1] : st.n[1] * st.n[2]);
+  const int bs = kStageThreads, pos = ND == 1 ? st.n[0] : (ND == 2 ? st.n[1] : st.n[1] * st.n[2]);
   const int nb = int(ceil_div(pos, bs));
   const int mi = ND == 1 ? 1 : planes_per_thread(st.n[0], (long long)nb * ne);
   const int ny = ND == 1 ? 1 : int(ceil_div(st.n[0], mi));
