@@ -231,8 +231,8 @@ def cpu_baseline(host, n, steps=5):
 def fp64_error(w, fp32_state, steps, torch):
     """Error of the FP32 headline run against an FP64 run of the same inputs: the
     FP32 advectee and advector promoted to FP64, advanced `steps` steps by the
-    FP64 fused kernel (the FP64 path equals the FP64 CPU restatement of the
-    reference to <= 1e-12), compared with the FP32 state after as many steps."""
+    FP64 path (which equals the FP64 CPU restatement of the reference to
+    <= 1e-12), compared with the FP32 state after as many steps."""
     from libmpdataxx_b200 import _lib
     w64 = {"grid": w["grid"], "advectee": [w["advectee"][0].double()], "advector": [a.double() for a in w["advector"]]}
     run = build_run(w64, "float64", torch)
@@ -243,7 +243,7 @@ def fp64_error(w, fp32_state, steps, torch):
     run.close()
     d = fp32_state.double() - out
     n = w["grid"][0]
-    return {"vs": "FP64 run of the same (FP32-rounded) inputs through the FP64 fused kernel", "after_steps": steps,
+    return {"vs": "FP64 run of the same (FP32-rounded) inputs through the FP64 path", "after_steps": steps,
             "max_abs": float(d.abs().max()), "l2": float(d.square().mean().sqrt()),
             "field_max": float(out.abs().max()), "cells": n ** 3}
 
@@ -294,9 +294,9 @@ def batched_extra(n_problems=256, steps=50):
 
 def box_1d_extra(steps=1000):
     """C1: 1D plain MPDATA (opts 0, n_iters 2), 2000 cyclic points, FP64, 1000 steps:
-    device time on the solver's stream (the general path: one kernel per formula
-    and halo fill, launch-bound at this size), mass and minimum after the run, and
-    the CPU restatement on the same set-up (one thread and all threads)."""
+    device time on the solver's stream (24 steps per launch in registers), mass and
+    minimum after the run, and the CPU restatement on the same set-up (one thread
+    and all threads)."""
     import numpy as np
     import torch
     sys.path.insert(0, os.path.join(ROOT, "oracle"))

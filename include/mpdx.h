@@ -53,8 +53,11 @@ enum { MPDX_PRS_CR = 0, MPDX_PRS_GCRK = 1 };
 enum { MPDX_PRECOND_IDENTITY = 0, MPDX_PRECOND_LEARNED = 1 };
 
 /* execution path: AUTO picks the fused kernels when the configuration allows
- * (all-cyclic, supported opts, periodic seams consistent) else GENERAL, which
- * runs one kernel per reference formula; both are CUDA. */
+ * (all-cyclic, supported opts, periodic seams consistent), or the staged step where
+ * that is faster (double precision in 3D, small grids), or several steps per launch in
+ * 1D; else, and under GENERAL, a step runs in a few launches of one stage each (opts
+ * within fct, iga and tot, up to three passes) or one kernel per reference formula.
+ * FUSED takes the fused kernels or fails.  All are CUDA. */
 enum { MPDX_PATH_AUTO = 0, MPDX_PATH_GENERAL = 1, MPDX_PATH_FUSED = 2 };
 
 /* field kinds for mpdx_set_field / mpdx_get_field */

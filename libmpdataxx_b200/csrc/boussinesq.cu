@@ -858,7 +858,8 @@ __device__ __forceinline__ bool grid_wait(unsigned *bar, unsigned target, int *t
     long long t0 = 0;
     ok = 1;
     for (;;) {
-      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      // (an acquire each time: a relaxed read and a fence after it took 0.5 us more per iteration)
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
       if (int(v - target) >= 0) break;
       const long long t = clock64();
       if (t0 == 0) t0 = t;
@@ -868,7 +869,6 @@ __device__ __forceinline__ bool grid_wait(unsigned *bar, unsigned target, int *t
         break;
       }
     }
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
   }
   __syncthreads();
   return ok != 0;
@@ -947,7 +947,11 @@ template <class T, int K, int R>
 __global__ void __launch_bounds__(kLoopThreads, 1)
     k_gcr_loop(geom g, T err_tol, dfield<T> phi, dfield<T> err0, dfield<T> err1, dfield<T> lap_err, dirs<T> D,
                gcr_dev<T> *dv, double2 *board, unsigned *bar, long long max_bodies) {
-  constexpr int U = R > 0 ? R : 2;  // points per pass
+  constexpr int U = R > 0 ? R : 2;   // points per pass of the first half
+  // and of the second, whose loads are all of the own points: as many as the registers
+  // hold with K directions (us per body with 2 and with this: K = 1 at 128 x 128 x 96 45.5
+  // and 42.6, K = 4 at 400 x 400 61.4 and 56.0)
+  constexpr int W = K == 1 ? 4 : (K < 4 ? 2 : 1);
   T alpha[K], tden[K];
 #pragma unroll
   for (int l = 0; l < K; ++l) { alpha[l] = dv->alpha[l]; tden[l] = dv->tmp_den[l]; }
@@ -976,6 +980,15 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
 #pragma unroll
     for (int d = 0; d < 3; ++d) c_now[d] = c_first[d];
   };
+  auto advance = [&] {
+    c_now[2] += dc[2];
+    int up = c_now[2] >= n2 ? 1 : 0;
+    c_now[2] -= up ? n2 : 0;
+    c_now[1] += dc[1] + up;
+    up = c_now[1] >= n1 ? 1 : 0;
+    c_now[1] -= up ? n1 : 0;
+    c_now[0] += dc[0] + up;
+  };
   int co[U][3], o[U];
   auto locate = [&](int q0) {  // the next U points (one beyond the last: the last one's values, unused)
 #pragma unroll
@@ -985,13 +998,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
       co[u][1] = d3 ? (in ? c_now[1] : 0) : (in ? c_now[2] : 0);
       co[u][2] = d3 && in ? c_now[2] : 0;
       o[u] = in ? c_now[0] * s0 + c_now[1] * s1 + c_now[2] : 0;
-      c_now[2] += dc[2];
-      int up = c_now[2] >= n2 ? 1 : 0;
-      c_now[2] -= up ? n2 : 0;
-      c_now[1] += dc[1] + up;
-      up = c_now[1] >= n1 ? 1 : 0;
-      c_now[1] -= up ? n1 : 0;
-      c_now[0] += dc[0] + up;
+      advance();
     }
   };
   __shared__ int4 t_off[kLapRows];
@@ -1064,37 +1071,44 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
       for (int l = 1; l < K; ++l)
         if (!restart && l == v + 1) { pd = D.p[l].o; lpd = D.lp[l].o; }
       dd bs[2] = {{0.0, 0.0}, {0.0, 0.0}};
-      if (R == 0) rewind();
-      for (int q0 = first; q0 < cells; q0 += U * nthr) {
-        if (R == 0) {
-          locate(q0);
+      auto second = [&](int oo, T ev, T lv, T pv, const T (&pp)[K], const T (&lp)[K]) {
+        T pn = ev, ln = lv;
 #pragma unroll
-          for (int u = 0; u < U; ++u) {
-            e[u] = ebo[o[u]];
-            le[u] = leo[o[u]];
-            ph[u] = phio[o[u]];
+        for (int l = 0; l < K; ++l)
+          if (l <= v) {
+            pn = pn + alpha[l] * pp[l];
+            ln = ln + alpha[l] * lp[l];
+            if (l == v) phio[oo] = pv + b * pp[l];
+          }
+        pd[oo] = pn;
+        lpd[oo] = ln;
+        bs[0] = dd_add(bs[0], dd{double(T(ln * ln)), 0.0});
+        bs[1] = dd_add(bs[1], dd{double(T(ev * ln)), 0.0});
+      };
+      if constexpr (R > 0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (first + u * nthr < cells) second(o[u], e[u], le[u], ph[u], po[u], lpo[u]);
+      } else {
+        rewind();
+        for (int q0 = first; q0 < cells; q0 += W * nthr) {
+          int oo[W];
+          T ev[W], lv[W], pv[W], pp[W][K], lp[W][K];
+#pragma unroll
+          for (int u = 0; u < W; ++u) {
+            oo[u] = q0 + u * nthr < cells ? c_now[0] * s0 + c_now[1] * s1 + c_now[2] : 0;
+            advance();
+            ev[u] = ebo[oo[u]];
+            lv[u] = leo[oo[u]];
+            pv[u] = phio[oo[u]];
 #pragma unroll
             for (int l = 0; l < K; ++l)
-              if (l <= v) { po[u][l] = D.p[l].o[o[u]]; lpo[u][l] = D.lp[l].o[o[u]]; }
+              if (l <= v) { pp[u][l] = D.p[l].o[oo[u]]; lp[u][l] = D.lp[l].o[oo[u]]; }
           }
-        }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (q0 + u * nthr >= cells) continue;
-          T pn = e[u], ln = le[u];
-#pragma unroll
-          for (int l = 0; l < K; ++l)
-            if (l <= v) {
-              pn = pn + alpha[l] * po[u][l];
-              ln = ln + alpha[l] * lpo[u][l];
-              if (l == v) phio[o[u]] = ph[u] + b * po[u][l];
-            }
-          pd[o[u]] = pn;
-          lpd[o[u]] = ln;
-          bs[0] = dd_add(bs[0], dd{double(T(ln * ln)), 0.0});
-          bs[1] = dd_add(bs[1], dd{double(T(e[u] * ln)), 0.0});
+          for (int u = 0; u < W; ++u)
+            if (q0 + u * nthr < cells) second(oo[u], ev[u], lv[u], pv[u], pp[u], lp[u]);
         }
-        if (R > 0) break;
       }
       double z0 = 0, z1 = 0;
       if (!all_reduce<2, false>(bs, 2, z0, z1, board, bar, epoch, &dv->timeout)) { alive = false; break; }
@@ -1568,11 +1582,12 @@ unsigned red_grid(const bq::geom &g) {
 // per inner step are taken instead: grids of more than kLoopCells points, where the
 // shared planes of k_gcr_update3 save more than the launches cost, and axes that do
 // not fit the table of index rules.  FP64, us per iteration of cr, two launches
-// against one: 48 x 48 19 and 7.0, 201 x 201 22 (38 with whole rows per warp) and 7.7,
-// 400 x 400 32 and 11.6, 1000 x 1000 56 and 26, 97 x 89 x 65 53 and 22, 128 x 128 x 96
-// 67 and 47, 160 x 160 x 96 (2.46 M points) 89 and 80; gcrk with k = 3 at 97 x 89 x 65
-// 178 and 87 per body.  512 threads with 128 registers and two points per pass: with
-// 1024 threads and 64 registers fewer loads are in flight (160 x 160 x 96: 120).
+// against one: 48 x 48 19 and 6.4, 201 x 201 22 (38 with whole rows per warp) and 7.2,
+// 400 x 400 32 and 10.8, 1000 x 1000 56 and 26, 97 x 89 x 65 53 and 20.6,
+// 128 x 128 x 96 67 and 42.6, 160 x 160 x 96 (2.46 M points) 89 and 73.5; gcrk with
+// k = 3 at 97 x 89 x 65 178 and 80.5 per body.  512 threads with 128 registers and two
+// points per pass: with 1024 threads and 64 registers fewer loads are in flight
+// (160 x 160 x 96: 120).
 struct loop_shape {
   int blocks, threads;
 };

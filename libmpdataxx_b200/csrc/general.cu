@@ -1,9 +1,10 @@
 // Reference-structured MPDATA path: one kernel per libmpdata++ formula and one
 // small kernel per halo fill, launched in the order the reference's solvers call
 // them.  It covers every dimension, the cyclic, open and rigid boundary conditions
-// and the MPDATA options that the fused kernels do not, and it is the FP64
-// parity path (this file is compiled with --fmad=false so that FP64 results
-// follow the reference's rounding).
+// and every MPDATA option built; steps within the common options (fct, iga, tot, up
+// to three passes) go to the staged kernels instead (stages_impl.cuh: the same
+// arithmetic in four launches).  Compiled with --fmad=false so that FP64 results
+// follow the reference's rounding.
 //
 // Reference call structure mirrored here:
 //   advop            libmpdata++/solvers/detail/mpdata_osc_{1,2,3}d.hpp

@@ -285,11 +285,19 @@ struct mpdata_solver : solver_base {
     if (st.nd == 3) return dbl || (st.cells() <= 1000000 && fused3d_planes_setting(-1) == 0);
     return dbl && st.cells() <= (st.n_iters == 3 ? 16000000 : 600000);
   }
+  // whether a 1D problem's ends allow several steps per launch; the check reads a flag
+  // back, so an advance that is being captured goes by the last check or does without
+  bool line_seams() {
+    if (st.bcs[0][0] != MPDX_BC_CYCLIC) return true;
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    MPDX_CUDA(cudaStreamIsCapturing(stream, &c));
+    if (c != cudaStreamCaptureStatusNone && fus.known < 0) return false;
+    return fus.seams_consistent(st, scratch);
+  }
   void advance(long long nt) override {
     if (nt <= 0) return;
     if (st.timestep == 0) gen.ante_loop(scratch);
-    if (path != MPDX_PATH_GENERAL && stage_engine<T>::line_covers(st) &&
-        (st.bcs[0][0] != MPDX_BC_CYCLIC || fus.seams_consistent(st, scratch))) {
+    if (path != MPDX_PATH_GENERAL && stage_engine<T>::line_covers(st) && line_seams()) {
       gen.stages.line(st, nt);
       last_path = MPDX_PATH_FUSED;
       return;

@@ -1077,7 +1077,7 @@ void stage_engine<T>::step(mpdata_state<T> &st, bool upwind_only) {
   for (int e0 = 0; e0 < st.n_eqns; e0 += most) {
     const int ne = std::min(most, st.n_eqns - e0);
     if (int(more.size()) < ne - 1) more.resize(ne - 1);
-    for (int q = 0; passes > 1 && q < ne - 1; ++q) {
+    for (int q = 0; st.n_iters > 1 && q < ne - 1; ++q) {
       auto &w = more[q];
       if (w.tmp0[0].base) continue;
       st.alloc_vctr(w.tmp0);
