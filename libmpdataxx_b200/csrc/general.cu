@@ -672,10 +672,9 @@ __global__ void k_zero_div(dfield<T> Ad, dfield<T> A1, dfield<T> A2, int nd, int
 
 // rigid walls (bcond/rigid_{2,3}d.hpp), halo position f + t, t in [0, cnt):
 //   mode 0 (scalar mirror):   A(f+t) = A(src0 + sgn*t)
-//   mode 1 (pressure):        A(f+t) = 2 A(edge) - A(src0 + sgn*t)
 //   mode 2 (negated mirror):  A(f+t) = -A(src0 + sgn*t)
 template <class T>
-__global__ void k_halo_rigid(dfield<T> A, int nd, int d, int mode, int f, int cnt, int src0, int sgn, int edge,
+__global__ void k_halo_rigid(dfield<T> A, int nd, int d, int mode, int f, int cnt, int src0, int sgn,
                              int bf, int nb, int cf, int nc) {
   const long long tot = (long long)cnt * nb * nc;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < tot; q += (long long)gridDim.x * blockDim.x) {
@@ -686,7 +685,6 @@ __global__ void k_halo_rigid(dfield<T> A, int nd, int d, int mode, int f, int cn
     const T m = PR(A, nd, d, src0 + sgn * t, b, c);
     T v;
     if (mode == 0) v = m;
-    else if (mode == 1) v = T(2) * PR(A, nd, d, edge, b, c) - m;
     else v = -m;
     PR(A, nd, d, f + t, b, c) = v;
   }
@@ -719,27 +717,11 @@ void general<T>::fill_sclr(int d, int side, field<T> &A, rng rb, rng rc, bool de
     k_halo_set<T><<<grid_for(tot), 256, 0, S.stream>>>(A.v, nd, d, f, H, e, !deriv, T(0), rb.f, rb.n(), rc.f, rc.n());
   } else if (kind == MPDX_BC_RIGID) {
     // mirror about the wall point: A(-m) = A(m), A(n-1+m) = A(n-1-m)  (rigid_2d.hpp:16-24, 124-132)
-    if (side == 0) k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(A.v, nd, d, 0, -H, H, H, -1, 0, rb.f, rb.n(), rc.f, rc.n());
-    else k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(A.v, nd, d, 0, n, H, n - 2, -1, 0, rb.f, rb.n(), rc.f, rc.n());
+    if (side == 0) k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(A.v, nd, d, 0, -H, H, H, -1, rb.f, rb.n(), rc.f, rc.n());
+    else k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(A.v, nd, d, 0, n, H, n - 2, -1, rb.f, rb.n(), rc.f, rc.n());
   } else {
     throw error(MPDX_E_UNSUPPORTED, "boundary condition not supported for scalars on this path");
   }
-  MPDX_LAUNCH_CHECK();
-}
-
-template <class T>
-void general<T>::fill_pres(int d, int side, field<T> &A, rng rb, rng rc) {
-  auto &S = *s;
-  const int kind = S.bcs[d][side];
-  if (kind == MPDX_BC_CYCLIC) { fill_sclr(d, side, A, rb, rc); return; }
-  if (kind != MPDX_BC_RIGID) throw error(MPDX_E_UNSUPPORTED, "boundary condition not supported for pressure on this path");
-  const int nd = S.nd, H = S.H, n = S.n[d];
-  if (nd < 2) rb = {0, 0};
-  if (nd < 3) rc = {0, 0};
-  const long long tot = (long long)H * rb.n() * rc.n();
-  // A(-m) = 2 A(0) - A(m);  A(n-1+m) = 2 A(n-1) - A(n-1-m)  (rigid_2d.hpp:26-35, 134-143)
-  if (side == 0) k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(A.v, nd, d, 1, -H, H, H, -1, 0, rb.f, rb.n(), rc.f, rc.n());
-  else k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(A.v, nd, d, 1, n, H, n - 2, -1, n - 1, rb.f, rb.n(), rc.f, rc.n());
   MPDX_LAUNCH_CHECK();
 }
 
@@ -764,8 +746,8 @@ void general<T>::fill_flux(int d, int side, field<T> *AV, rng rb, rng rc) {
   if (nd < 3) rc = {0, 0};
   // F(-1) = -F(0);  F(n-1) = -F(n-2)  (rigid_2d.hpp:74-79, 170-175)
   const long long tot = (long long)rb.n() * rc.n();
-  if (side == 0) k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(AV[d].v, nd, d, 2, -1, 1, 0, 1, 0, rb.f, rb.n(), rc.f, rc.n());
-  else k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(AV[d].v, nd, d, 2, n - 1, 1, n - 2, 1, 0, rb.f, rb.n(), rc.f, rc.n());
+  if (side == 0) k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(AV[d].v, nd, d, 2, -1, 1, 0, 1, rb.f, rb.n(), rc.f, rc.n());
+  else k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(AV[d].v, nd, d, 2, n - 1, 1, n - 2, 1, rb.f, rb.n(), rc.f, rc.n());
   MPDX_LAUNCH_CHECK();
 }
 
@@ -785,7 +767,7 @@ void general<T>::fill_vctr_nrml(int d, int side, field<T> &A, rng rb, rng rc) {
 }
 
 template <class T>
-void general<T>::fill_vctr_alng(int d, int side, field<T> *AV, rng rb, rng rc, bool ad, bool cyclic_only) {
+void general<T>::fill_vctr_alng(int d, int side, field<T> *AV, rng rb, rng rc, bool ad) {
   auto &S = *s;
   const int kind = S.bcs[d][side];
   const int nd = S.nd, H = S.H, n = S.n[d];
@@ -799,7 +781,6 @@ void general<T>::fill_vctr_alng(int d, int side, field<T> *AV, rng rb, rng rc, b
     MPDX_LAUNCH_CHECK();
     return;
   }
-  if (cyclic_only) return;
   if (kind == MPDX_BC_RIGID) {
     // zero normal velocity at the wall point (rigid_2d.hpp:58-66, 154-162):
     // left  GC(-m) = -GC(m-1) for m = H .. 1 (.. 2 with ad);
@@ -807,8 +788,8 @@ void general<T>::fill_vctr_alng(int d, int side, field<T> *AV, rng rb, rng rc, b
     const int a = ad ? 1 : 0;
     const long long tot = (long long)(H - a) * rb.n() * rc.n();
     if (H - a > 0) {
-      if (side == 0) k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(AV[d].v, nd, d, 2, -H, H - a, H - 1, -1, 0, rb.f, rb.n(), rc.f, rc.n());
-      else k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(AV[d].v, nd, d, 2, n - 1 + a, H - a, n - 2, -1, 0, rb.f, rb.n(), rc.f, rc.n());
+      if (side == 0) k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(AV[d].v, nd, d, 2, -H, H - a, H - 1, -1, rb.f, rb.n(), rc.f, rc.n());
+      else k_halo_rigid<T><<<grid_for(tot), 256, 0, S.stream>>>(AV[d].v, nd, d, 2, n - 1 + a, H - a, n - 2, -1, rb.f, rb.n(), rc.f, rc.n());
       MPDX_LAUNCH_CHECK();
     }
     return;
@@ -870,19 +851,19 @@ void general<T>::xchng_sclr(field<T> &A, int ex, bool deriv) {
 }
 
 template <class T>
-void general<T>::xchng_vctr_alng(field<T> *AV, bool ad, bool cyclic) {
+void general<T>::xchng_vctr_alng(field<T> *AV, bool ad) {
   auto &S = *s;
   const rng *ir = S.ir;
-  if (S.nd == 1) { for (int q = 0; q < 2; ++q) fill_vctr_alng(0, q, AV, {0, 0}, {0, 0}, ad, cyclic); return; }
+  if (S.nd == 1) { for (int q = 0; q < 2; ++q) fill_vctr_alng(0, q, AV, {0, 0}, {0, 0}, ad); return; }
   if (S.nd == 2) {  // solver_2d.hpp:63-88
-    for (int q = 0; q < 2; ++q) fill_vctr_alng(0, q, AV, ir[1], {0, 0}, ad, cyclic);
-    for (int q = 0; q < 2; ++q) fill_vctr_alng(1, q, AV, ir[0], {0, 0}, ad, cyclic);
+    for (int q = 0; q < 2; ++q) fill_vctr_alng(0, q, AV, ir[1], {0, 0}, ad);
+    for (int q = 0; q < 2; ++q) fill_vctr_alng(1, q, AV, ir[0], {0, 0}, ad);
     return;
   }
   // solver_3d.hpp:73-103
-  for (int q = 0; q < 2; ++q) fill_vctr_alng(0, q, AV, ir[1], ir[2], ad, cyclic);
-  for (int q = 0; q < 2; ++q) fill_vctr_alng(1, q, AV, ir[2], ir[0], ad, cyclic);
-  for (int q = 0; q < 2; ++q) fill_vctr_alng(2, q, AV, ir[0], ir[1], ad, cyclic);
+  for (int q = 0; q < 2; ++q) fill_vctr_alng(0, q, AV, ir[1], ir[2], ad);
+  for (int q = 0; q < 2; ++q) fill_vctr_alng(1, q, AV, ir[2], ir[0], ad);
+  for (int q = 0; q < 2; ++q) fill_vctr_alng(2, q, AV, ir[0], ir[1], ad);
 }
 
 template <class T>
@@ -917,21 +898,6 @@ void general<T>::xchng_flux(field<T> *AV) {  // solver_2d.hpp:90-101, solver_3d.
   for (int q = 0; q < 2; ++q) fill_flux(0, q, AV, ir[1], ir[2]);
   for (int q = 0; q < 2; ++q) fill_flux(1, q, AV, ir[2], ir[0]);
   for (int q = 0; q < 2; ++q) fill_flux(2, q, AV, ir[0], ir[1]);
-}
-
-template <class T>
-void general<T>::xchng_pres(field<T> &A, int ex) {  // solver_2d.hpp:204-220, solver_3d.hpp:288-307
-  auto &S = *s;
-  const rng *ir = S.ir;
-  if (S.nd == 1) { for (int q = 0; q < 2; ++q) fill_pres(0, q, A, {0, 0}, {0, 0}); return; }
-  if (S.nd == 2) {
-    for (int q = 0; q < 2; ++q) fill_pres(0, q, A, ext(ir[1], ex), {0, 0});
-    for (int q = 0; q < 2; ++q) fill_pres(1, q, A, ext(ir[0], ex), {0, 0});
-    return;
-  }
-  for (int q = 0; q < 2; ++q) fill_pres(0, q, A, ext(ir[1], ex), ext(ir[2], ex));
-  for (int q = 0; q < 2; ++q) fill_pres(1, q, A, ext(ir[2], ex), ext(ir[0], ex));
-  for (int q = 0; q < 2; ++q) fill_pres(2, q, A, ext(ir[0], ex), ext(ir[1], ex));
 }
 
 template <class T>
