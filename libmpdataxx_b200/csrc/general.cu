@@ -10,6 +10,7 @@
 //   advop            libmpdata++/solvers/detail/mpdata_osc_{1,2,3}d.hpp
 //   fct_init / fct_adjust_antidiff   mpdata_fct_{1,2,3}d.hpp
 //   halo exchanges   solvers/detail/solver_{1,2,3}d.hpp, bcond/{cyclic,open,rigid}_{1,2,3}d.hpp
+#include <algorithm>
 #include <cfloat>
 
 #include "general.cuh"
@@ -1090,6 +1091,48 @@ void general<T>::ante_loop(double *dev_scratch) {
   }
   if (S.opts & o_nug) xchng_sclr(S.G, S.H);  // mpdata_osc_{1,2,3}d.hpp hook_ante_loop
   if (S.nd > 1) xchng_vctr_nrml(S.GC, S.H - 1);
+}
+
+// Halos of an advector on an all-cyclic grid with consistent seams: faces -H .. -1 and
+// n-1 .. n-2+H of a component along its own axis, points -H .. -1 and n .. n-1+H across,
+// corners included, each from its wrapped interior place: what xchng_vctr_alng and
+// xchng_vctr_nrml leave there, in one launch instead of 18 in 3D.  The halo points of
+// axis q: 2 H positions along q, interior positions along the axes before it, all
+// positions along those after it.
+template <class T>
+__global__ void k_wrap_advector(dfield<T> g0, dfield<T> g1, dfield<T> g2, int nd, int n0, int n1, int n2, int H) {
+  const int d = blockIdx.y, n[3] = {n0, n1, n2};
+  const dfield<T> g = d == 0 ? g0 : (d == 1 ? g1 : g2);
+  for (int q = 0; q < nd; ++q) {
+    int cnt[3] = {1, 1, 1}, low[3] = {0, 0, 0};
+    for (int a = 0; a < nd; ++a) {
+      const int in = a == d ? n[a] - 1 : n[a];
+      cnt[a] = a == q ? 2 * H : (a < q ? in : in + 2 * H);
+      low[a] = a < q ? 0 : -H;
+    }
+    const long long tot = (long long)cnt[0] * cnt[1] * cnt[2];
+    for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < tot; w += (long long)gridDim.x * blockDim.x) {
+      const long long r = w / cnt[2];
+      int c[3] = {low[0] + int(r / cnt[1]), low[1] + int(r % cnt[1]), low[2] + int(w % cnt[2])}, s[3];
+      if (c[q] >= 0) c[q] += q == d ? n[q] - 1 : n[q];  // the upper half of the 2 H positions
+      for (int a = 0; a < 3; ++a) {
+        const int P = n[a] - 1;
+        s[a] = a >= nd ? 0 : (c[a] < 0 ? c[a] + P : (c[a] > (a == d ? P - 1 : P) ? c[a] - P : c[a]));
+      }
+      g(c[0], c[1], c[2]) = g(s[0], s[1], s[2]);
+    }
+  }
+}
+
+template <class T>
+void general<T>::wrap_advector() {
+  auto &S = *s;
+  long long most = 0;  // halo points of the largest axis
+  for (int d = 0; d < S.nd; ++d) most = std::max(most, 2LL * S.H * (S.cells() / S.n[d]));
+  const dfield<T> z = S.GC[0].v;
+  k_wrap_advector<T><<<dim3(grid_for(most), S.nd), 256, 0, S.stream>>>(z, S.nd > 1 ? S.GC[1].v : z, S.nd > 2 ? S.GC[2].v : z,
+                                                                     S.nd, S.n[0], S.n[1], S.n[2], S.H);
+  MPDX_LAUNCH_CHECK();
 }
 
 template <class T>

@@ -144,7 +144,7 @@ struct solver_base {
   virtual void get_field(int kind, int idx, void *dst, bool device) = 0;
   virtual void view_extent(int kind, int idx, int ex[3]) = 0;
   virtual view_desc describe(int kind, int idx) = 0;
-  virtual void invalidate_fused() {}
+  virtual void field_written(int /*kind*/) {}  // by an asynchronous upload
   virtual void advance(long long nt) = 0;
   virtual void stats(mpdx_step_stats *out) = 0;
   // learned GCR preconditioner (Boussinesq solvers only)
@@ -206,6 +206,7 @@ struct mpdata_solver : solver_base {
   stats_engine<T> stat;
   fused_engine<T> fus;
   int path = MPDX_PATH_AUTO, last_path = MPDX_PATH_GENERAL;
+  bool new_advector = false;  // written since its halos were filled
   double *scratch = nullptr;
 
   mpdata_solver(const mpdx_config &c) {
@@ -259,12 +260,15 @@ struct mpdata_solver : solver_base {
     d.st[0] = f->v.s0; d.st[1] = f->v.s1; d.st[2] = f->v.s2;
     return d;
   }
-  void invalidate_fused() override { fus.invalidate(); }
+  void field_written(int kind) override {
+    fus.invalidate();
+    if (kind == MPDX_FIELD_ADVECTOR) new_advector = true;
+  }
   void set_field(int kind, int idx, const void *src, bool device) override {
     int ex[3], off[3]; field<T> *f;
     view(kind, idx, ex, off, f);
     xfer.put(stream, *f, src, device, ex, off);
-    fus.invalidate();
+    field_written(kind);
   }
   void get_field(int kind, int idx, void *dst, bool device) override {
     int ex[3], off[3]; field<T> *f;
@@ -289,14 +293,34 @@ struct mpdata_solver : solver_base {
   // back, so an advance that is being captured goes by the last check or does without
   bool line_seams() {
     if (st.bcs[0][0] != MPDX_BC_CYCLIC) return true;
+    if (capturing() && fus.known < 0) return false;
+    return fus.seams_consistent(st, scratch);
+  }
+  // before the first step: the advector's halos are filled (here and nowhere else, as
+  // the reference does, for the steps that follow the reference's halo rules) and its
+  // divergence checked
+  void ante_loop() {
+    if (st.timestep != 0) return;
+    gen.ante_loop(scratch);
+    new_advector = false;
+  }
+  bool capturing() const {
     cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
     MPDX_CUDA(cudaStreamIsCapturing(stream, &c));
-    if (c != cudaStreamCaptureStatusNone && fus.known < 0) return false;
-    return fus.seams_consistent(st, scratch);
+    return c != cudaStreamCaptureStatusNone;
+  }
+  // The fused kernels wrap their indices; the stages read the advector's halos, which
+  // are brought up to date before they take the fused kernels' place.  A captured
+  // advance does so in every replay: new advectors may be uploaded between replays.
+  void refresh_advector() {
+    const bool cap = capturing();
+    if (!cap && !new_advector) return;
+    gen.wrap_advector();
+    if (!cap) new_advector = false;
   }
   void advance(long long nt) override {
     if (nt <= 0) return;
-    if (st.timestep == 0) gen.ante_loop(scratch);
+    ante_loop();
     if (path != MPDX_PATH_GENERAL && stage_engine<T>::line_covers(st) && line_seams()) {
       gen.stages.line(st, nt);
       last_path = MPDX_PATH_FUSED;
@@ -316,6 +340,7 @@ struct mpdata_solver : solver_base {
     }
     last_path = use_fused ? MPDX_PATH_FUSED : MPDX_PATH_GENERAL;
     const bool one_kernel = use_fused && !(path == MPDX_PATH_AUTO && stages_faster());
+    if (use_fused && !one_kernel) refresh_advector();
     for (long long t = 0; t < nt; ++t) {
       if (one_kernel) fus.step(st);
       else gen.step();
@@ -547,7 +572,7 @@ struct batch_impl : batch_base {
       h->xfer_async->join(h->stream);
       MPDX_CUDA(cudaStreamSynchronize(h->stream));
       try {
-        if (h->st.timestep == 0) h->gen.ante_loop(h->scratch);
+        h->ante_loop();
       } catch (const error &e) {
         throw error(e.code, std::string(e.what()) + " (batch problem " + std::to_string(p) + ")");
       }
@@ -863,7 +888,7 @@ mpdx_status mpdx_set_field_async(mpdx_handle h, int kind, int idx, const void *h
     if (!host) throw mpdx::error(MPDX_E_ARG, "null host buffer");
     const auto v = h->impl->describe(kind, idx);
     h->impl->xfer_async->transfer(h->impl->stream, kind, idx, v, const_cast<void *>(host), h->impl->dtype, true);
-    h->impl->invalidate_fused();
+    h->impl->field_written(kind);
   });
 }
 
