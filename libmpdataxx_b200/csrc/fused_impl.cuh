@@ -239,7 +239,8 @@ int fused2d_batched(int tile, int ni, bool iga, bool fct, const f2::prob<T> *pro
 
 // ---------------------------------------------------------------------------
 // seam check: the duplicate point n-1 must equal point 0 along every periodic
-// axis, for the advectees and for the transverse axes of the advector faces.
+// axis, for the advectees and for the transverse axes of the advector faces (and, in
+// 1D, for the faces at the ends).
 template <class T>
 __device__ __forceinline__ bool same_bits(T a, T b) {
   if (sizeof(T) == 8) return __double_as_longlong(double(a)) == __double_as_longlong(double(b));
@@ -262,6 +263,13 @@ __global__ void k_seam(dfield<T> f, int ax, int last, int e0, int e1, int e2, un
   }
 }
 
+// one-dimensional: the faces beyond the unique ones repeat those they stand for (an
+// advector set after the first step brings its own face -1 and leaves face n-1)
+template <class T>
+__global__ void k_seam_faces(dfield<T> g, int n, unsigned *flag) {
+  if (!same_bits(g(-1, 0, 0), g(n - 2, 0, 0)) || !same_bits(g(n - 1, 0, 0), g(0, 0, 0))) *flag = 1u;
+}
+
 template <class T>
 bool fused_seams_consistent(mpdata_state<T> &st, double *scratch) {
   unsigned *flag = reinterpret_cast<unsigned *>(scratch);
@@ -282,6 +290,10 @@ bool fused_seams_consistent(mpdata_state<T> &st, double *scratch) {
   for (int d = 0; d < st.nd; ++d)
     for (int ax = 0; ax < st.nd; ++ax)
       if (ax != d) check(st.GC[d], ax, d);
+  if (st.nd == 1) {
+    k_seam_faces<T><<<1, 1, 0, st.stream>>>(st.GC[0].v, st.n[0], flag);
+    MPDX_LAUNCH_CHECK();
+  }
   unsigned h = 0;
   MPDX_CUDA(cudaMemcpyAsync(&h, flag, sizeof(h), cudaMemcpyDeviceToHost, st.stream));
   MPDX_CUDA(cudaStreamSynchronize(st.stream));

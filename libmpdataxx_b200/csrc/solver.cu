@@ -289,12 +289,11 @@ struct mpdata_solver : solver_base {
     if (st.nd == 3) return dbl || (st.cells() <= 1000000 && fused3d_planes_setting(-1) == 0);
     return dbl && st.cells() <= (st.n_iters == 3 ? 16000000 : 600000);
   }
-  // whether a 1D problem's ends allow several steps per launch; the check reads a flag
-  // back, so an advance that is being captured goes by the last check or does without
+  // whether a 1D problem's ends allow several steps per launch.  Not in an advance that
+  // is being captured: the fields at its replays may be others.
   bool line_seams() {
     if (st.bcs[0][0] != MPDX_BC_CYCLIC) return true;
-    if (capturing() && fus.known < 0) return false;
-    return fus.seams_consistent(st, scratch);
+    return !capturing() && fus.seams_consistent(st, scratch);
   }
   // before the first step: the advector's halos are filled (here and nowhere else, as
   // the reference does, for the steps that follow the reference's halo rules) and its

@@ -4,7 +4,8 @@ that was set last, halos included: the same fields as a handle made anew for eac
 (bit for bit) and as the fused kernels, which wrap their indices (FP64 3D bit for bit;
 FP64 2D 1e-12 and FP32 1e-5 of the field's maximum, whose arithmetic differs in
 rounding).  Uploads by the synchronous and asynchronous calls and from device memory,
-and between the replays of a captured advance."""
+and between the replays of a captured advance.  In 1D the halos are filled before the
+first step only, as in the reference, on every path."""
 import numpy as np
 import pytest
 import torch
@@ -109,3 +110,23 @@ def test_new_advector_between_replays(grid, opts, iters, dtype):
     fresh.advance(1)
     np.testing.assert_array_equal(np.array(run.advectee()), fresh.advectee())
     del g
+
+
+@pytest.mark.parametrize("bc", ["cyclic", "open"])
+@pytest.mark.parametrize("opts,n_eqns", [(0, 1), (o.iga | o.fct, 1), (o.fct, 2)])
+def test_new_advector_1d_as_general(opts, n_eqns, bc):
+    n, rng = 70, np.random.default_rng(4)
+    psi = [rng.uniform(0.5, 2.0, n) for _ in range(n_eqns)]
+    for a in psi:
+        a[-1] = a[0]
+    runs = [make_run((n,), opts, n_eqns=n_eqns, bcs=[bc] * 2, path=p) for p in ("general", "auto")]
+    for k in range(3):
+        c = rng.uniform(0.1, 0.4, n) if k else np.full(n, 0.3)
+        for r in runs:
+            for e, a in enumerate(psi):
+                if k == 0:
+                    r.set_advectee(a, e)
+            r.set_advector(c, 0)
+            r.advance(5)
+        for e in range(n_eqns):
+            np.testing.assert_array_equal(np.array(runs[1].advectee(e)), runs[0].advectee(e))
