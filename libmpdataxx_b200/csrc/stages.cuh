@@ -17,11 +17,14 @@ struct stage_engine {
     field<T> tmp0[3], tmp1[3], beta_up, beta_dn, psi_min, psi_max;
   };
   std::vector<work> more;
+  bool more_ready = false, one_by_one = false;  // `more` is allocated; it could not be
 
   // whether step() covers the configuration
   static bool covers(const mpdata_state<T> &st);
   // advances every equation by one step; `upwind_only`: the first pass alone
   void step(mpdata_state<T> &st, bool upwind_only);
+  // equations that one launch takes
+  int together(mpdata_state<T> &st);
   // one-dimensional problems with both ends open, or cyclic with consistent seams:
   // nt steps, several per launch (advances st.timestep)
   static bool line_covers(const mpdata_state<T> &st);

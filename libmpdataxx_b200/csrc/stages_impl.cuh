@@ -1070,21 +1070,42 @@ void stage_engine<T>::line(mpdata_state<T> &st, long long nt) {
 // together stay in cache and the launches count), one of a large grid.
 constexpr long long kStageBatchCells = 1 << 18;
 
+// The further work arrays are made by the first step that has a use for them.  A step
+// that is being captured cannot allocate, and goes equation by equation if it is the
+// first; so does every step where memory is short.
 template <class T>
-void stage_engine<T>::step(mpdata_state<T> &st, bool upwind_only) {
-  const int passes = upwind_only ? 1 : st.n_iters;
-  const int most = st.cells() <= kStageBatchCells ? kStageEqns : 1;
-  for (int e0 = 0; e0 < st.n_eqns; e0 += most) {
-    const int ne = std::min(most, st.n_eqns - e0);
-    if (int(more.size()) < ne - 1) more.resize(ne - 1);
-    for (int q = 0; st.n_iters > 1 && q < ne - 1; ++q) {
-      auto &w = more[q];
-      if (w.tmp0[0].base) continue;
+int stage_engine<T>::together(mpdata_state<T> &st) {
+  const int most = std::min(kStageEqns, st.n_eqns);
+  if (most == 1 || st.cells() > kStageBatchCells || one_by_one) return 1;
+  if (more_ready) return most;
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  MPDX_CUDA(cudaStreamIsCapturing(st.stream, &c));
+  if (c != cudaStreamCaptureStatusNone) return 1;
+  try {
+    more.resize(most - 1);
+    for (auto &w : more) {
+      if (st.n_iters == 1) break;  // an upwind pass has no work arrays
       st.alloc_vctr(w.tmp0);
       if (st.n_iters > 2) st.alloc_vctr(w.tmp1);
       if (st.opts & o_fct)
         for (field<T> *f : {&w.beta_up, &w.beta_dn, &w.psi_min, &w.psi_max}) st.alloc_sclr(*f);
     }
+  } catch (const error &) {
+    (void)cudaGetLastError();
+    more.clear();
+    one_by_one = true;
+    return 1;
+  }
+  more_ready = true;
+  return most;
+}
+
+template <class T>
+void stage_engine<T>::step(mpdata_state<T> &st, bool upwind_only) {
+  const int passes = upwind_only ? 1 : st.n_iters;
+  const int most = together(st);
+  for (int e0 = 0; e0 < st.n_eqns; e0 += most) {
+    const int ne = std::min(most, st.n_eqns - e0);
     if (st.nd == 1) sg::step_nd<T, 1>(st, *this, e0, ne, passes);
     else if (st.nd == 2) sg::step_nd<T, 2>(st, *this, e0, ne, passes);
     else sg::step_nd<T, 3>(st, *this, e0, ne, passes);
