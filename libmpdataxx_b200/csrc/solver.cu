@@ -269,6 +269,8 @@ struct mpdata_solver : solver_base {
     view(kind, idx, ex, off, f);
     xfer.put(stream, *f, src, device, ex, off);
     field_written(kind);
+    // this call waits for the device anyway; advance() does not after the first step
+    if (st.timestep > 0 && line_cyclic()) fus.seams_consistent(st, scratch);
   }
   void get_field(int kind, int idx, void *dst, bool device) override {
     int ex[3], off[3]; field<T> *f;
@@ -289,11 +291,17 @@ struct mpdata_solver : solver_base {
     if (st.nd == 3) return dbl || (st.cells() <= 1000000 && fused3d_planes_setting(-1) == 0);
     return dbl && st.cells() <= (st.n_iters == 3 ? 16000000 : 600000);
   }
+  bool line_cyclic() const {
+    return path != MPDX_PATH_GENERAL && stage_engine<T>::line_covers(st) && st.bcs[0][0] == MPDX_BC_CYCLIC;
+  }
   // whether a 1D problem's ends allow several steps per launch.  Not in an advance that
-  // is being captured: the fields at its replays may be others.
+  // is being captured: the fields at its replays may be others.  Nor where the check,
+  // which reads a flag back, would have this call wait after the first step (an
+  // asynchronous upload came before it).
   bool line_seams() {
-    if (st.bcs[0][0] != MPDX_BC_CYCLIC) return true;
-    return !capturing() && fus.seams_consistent(st, scratch);
+    if (!line_cyclic()) return true;
+    if (capturing() || (fus.known < 0 && st.timestep > 0)) return false;
+    return fus.seams_consistent(st, scratch);
   }
   // before the first step: the advector's halos are filled (here and nowhere else, as
   // the reference does, for the steps that follow the reference's halo rules) and its

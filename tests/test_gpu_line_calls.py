@@ -1,6 +1,8 @@
 """Calls on one-dimensional problems that the kernel of several steps per launch must
 leave as they are: a first advance under stream capture, which has no room for
-allocations."""
+allocations, and an advance after an upload, which returns before the device is done."""
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -43,3 +45,28 @@ def test_first_advance_captured(opts, n_eqns, iters, bc):
     for e in range(n_eqns):
         np.testing.assert_array_equal(np.array(run.advectee(e)), ref.advectee(e))
     del g
+
+
+@pytest.mark.parametrize("kind", ["sync", "async"])
+def test_advance_after_upload_does_not_wait(kind):
+    """The device is busy for about half a second when advance() is called."""
+    ref, run = pair(3000, o.iga | o.fct, 1)
+    for r in (ref, run):
+        r.advance(2)
+        r.sync()
+    a = torch.from_numpy(np.array(ref.advectee())[::-1].copy()).pin_memory()
+    if kind == "sync":
+        run.set_advectee(a.numpy())
+    else:
+        run.set_field_async(_lib.FIELD_ADVECTEE, 0, a.data_ptr())
+    with torch.cuda.stream(torch.cuda.ExternalStream(run.stream)):
+        torch.cuda._sleep(1 << 30)
+    t = time.perf_counter()
+    assert run.L.mpdx_advance(run.h, 3) == _lib.MPDX_OK
+    returned = time.perf_counter() - t
+    run.sync()
+    waited = time.perf_counter() - t
+    assert waited > 0.3 and returned < 0.1 * waited, (returned, waited)
+    ref.set_advectee(a.numpy())
+    ref.advance(3)
+    np.testing.assert_array_equal(np.array(run.advectee()), ref.advectee())
