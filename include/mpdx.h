@@ -60,6 +60,12 @@ enum { MPDX_PRECOND_IDENTITY = 0, MPDX_PRECOND_LEARNED = 1 };
  * FUSED takes the fused kernels or fails.  All are CUDA. */
 enum { MPDX_PATH_AUTO = 0, MPDX_PATH_GENERAL = 1, MPDX_PATH_FUSED = 2 };
 
+/* kernels that a step runs (mpdx_step_stats.kernels): none yet; one kernel per formula
+ * and halo fill; one launch per stage; the fused kernel; several 1D steps per launch in
+ * registers; all 1D steps of a call in one block */
+enum { MPDX_KERNELS_NONE = 0, MPDX_KERNELS_FORMULAS = 1, MPDX_KERNELS_STAGES = 2, MPDX_KERNELS_FUSED = 3,
+       MPDX_KERNELS_LINE = 4, MPDX_KERNELS_BLOCK = 5 };
+
 /* field kinds for mpdx_set_field / mpdx_get_field */
 enum {
   MPDX_FIELD_ADVECTEE = 0,   /* idx = equation; interior n0 x n1 x n2 */
@@ -114,10 +120,13 @@ typedef struct {
   int64_t gcr_iters;       /* iterations of the last pressure solve (Boussinesq) */
   int64_t gcr_iters_total; /* since creation */
   double gcr_residual;     /* max|err| at the end of the last pressure solve */
-  int path;                /* path used by the last advance (MPDX_PATH_GENERAL/FUSED) */
+  int path;                /* MPDX_PATH_FUSED where the last advance met the fused path's conditions (periodic
+                              options and seams; 1D: those of the one-block kernel), whichever kernels
+                              the automatic path then took (`kernels`), else MPDX_PATH_GENERAL */
   double gcr_ms;           /* device time of the last pressure solve, start to max|err| <= prs_tol / dt */
   int gcr_fallback;        /* 1 if the last solve left the learned preconditioner for plain GCR,
                               2 if it was redone from its start with plain GCR alone */
+  int kernels;             /* MPDX_KERNELS_* of the last advance */
 } mpdx_step_stats;
 
 /* Fill *cfg with the reference defaults (opts = iga|fct, n_iters = 2, ...). */

@@ -18,6 +18,7 @@ SOLVER_MPDATA, SOLVER_BOUSSINESQ = 0, 1
 PRS_CR, PRS_GCRK = 0, 1
 PRECOND_IDENTITY, PRECOND_LEARNED = 0, 1
 PATH_AUTO, PATH_GENERAL, PATH_FUSED = 0, 1, 2
+KERNELS_NONE, KERNELS_FORMULAS, KERNELS_STAGES, KERNELS_FUSED, KERNELS_LINE, KERNELS_BLOCK = range(6)
 FIELD_ADVECTEE, FIELD_ADVECTOR, FIELD_SCLR_ARRAY, FIELD_PRESSURE, FIELD_G = 0, 1, 2, 3, 4
 SCLR_THT_E = 0
 SCLR_THT_ABS = 1
@@ -57,7 +58,7 @@ class StepStats(ctypes.Structure):
     _fields_ = [("timestep", ctypes.c_int64), ("time", ctypes.c_double), ("mass", ctypes.c_double),
                 ("min", ctypes.c_double), ("max", ctypes.c_double), ("gcr_iters", ctypes.c_int64),
                 ("gcr_iters_total", ctypes.c_int64), ("gcr_residual", ctypes.c_double), ("path", ctypes.c_int),
-                ("gcr_ms", ctypes.c_double), ("gcr_fallback", ctypes.c_int)]
+                ("gcr_ms", ctypes.c_double), ("gcr_fallback", ctypes.c_int), ("kernels", ctypes.c_int)]
 
 
 class Tuning3D(ctypes.Structure):

@@ -22,6 +22,7 @@ struct general {
   void init_g();
   // one time step of every equation (solver_common.hpp:127-136, 321-331)
   void step();
+  int kernels() const { return stage_engine<T>::covers(*s) ? MPDX_KERNELS_STAGES : MPDX_KERNELS_FORMULAS; }
   // nt steps of a small cyclic 1D problem (one equation; no fct, dfl, nug or
   // divergence form) in one launch of one block, with step()'s arithmetic
   bool block1d_ok() const;

@@ -205,7 +205,7 @@ struct mpdata_solver : solver_base {
   transfer<T> xfer;
   stats_engine<T> stat;
   fused_engine<T> fus;
-  int path = MPDX_PATH_AUTO, last_path = MPDX_PATH_GENERAL;
+  int path = MPDX_PATH_AUTO, last_path = MPDX_PATH_GENERAL, last_kernels = MPDX_KERNELS_NONE;
   bool new_advector = false;  // written since its halos were filled
   double *scratch = nullptr;
 
@@ -330,13 +330,15 @@ struct mpdata_solver : solver_base {
     ante_loop();
     if (path != MPDX_PATH_GENERAL && stage_engine<T>::line_covers(st) && line_seams()) {
       gen.stages.line(st, nt);
-      last_path = MPDX_PATH_FUSED;
+      last_path = gen.block1d_ok() ? MPDX_PATH_FUSED : MPDX_PATH_GENERAL;
+      last_kernels = MPDX_KERNELS_LINE;
       return;
     }
     if (path != MPDX_PATH_GENERAL && gen.block1d_ok()) {
       gen.block1d(nt);
       st.timestep += nt;
       last_path = MPDX_PATH_FUSED;
+      last_kernels = MPDX_KERNELS_BLOCK;
       return;
     }
     bool use_fused = false;
@@ -347,6 +349,7 @@ struct mpdata_solver : solver_base {
     }
     last_path = use_fused ? MPDX_PATH_FUSED : MPDX_PATH_GENERAL;
     const bool one_kernel = use_fused && !(path == MPDX_PATH_AUTO && stages_faster());
+    last_kernels = one_kernel ? MPDX_KERNELS_FUSED : gen.kernels();
     if (use_fused && !one_kernel) refresh_advector();
     for (long long t = 0; t < nt; ++t) {
       if (one_kernel) fus.step(st);
@@ -359,6 +362,7 @@ struct mpdata_solver : solver_base {
     out->timestep = st.timestep;
     stat.reduce(st, st.psi[0][st.tl[0]], out);
     out->path = last_path;
+    out->kernels = last_kernels;
   }
   void tuning3d(mpdx_tuning3d *out) override {
     std::memset(out, 0, sizeof(*out));
@@ -466,6 +470,7 @@ struct boussinesq_solver : solver_base {
     out->gcr_ms = b->last_solve_ms;
     out->gcr_fallback = b->restarted ? 2 : (b->fell_back ? 1 : 0);
     out->path = MPDX_PATH_GENERAL;
+    out->kernels = st.timestep > 0 ? b->gen.kernels() : int(MPDX_KERNELS_NONE);
   }
 };
 
@@ -637,6 +642,7 @@ struct batch_impl : batch_base {
     for (auto *h : hs) {
       h->st.timestep += nt;
       h->last_path = MPDX_PATH_FUSED;
+      h->last_kernels = MPDX_KERNELS_FUSED;
     }
     MPDX_CUDA(cudaEventRecord(ev_done, stream));
     for (auto *h : hs) MPDX_CUDA(cudaStreamWaitEvent(h->stream, ev_done, 0));
