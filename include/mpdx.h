@@ -194,7 +194,10 @@ int mpdx_fused3d_bulk_copies(int mode);
  * 512); a negative value only queries.  Returns the setting before the call, or
  * -1 for an invalid value (which changes nothing).  Every value gives
  * bitwise-identical fields: a point is computed by the same operations whichever
- * CTA holds it.  No reference counterpart (the reference's threads split the
+ * CTA holds it.  It holds for the handles that take the fused 3D kernel: those on
+ * MPDX_PATH_FUSED, and on the automatic path in single precision above 10^6 points and
+ * in double precision while a positive value is set (otherwise a double precision
+ * handle steps in stages there, with the same bits).  No reference counterpart (the reference's threads split the
  * domain along x by its own rule, concurr/detail/concurr_common.hpp). */
 int mpdx_fused3d_planes_per_cta(int lx);
 
@@ -204,7 +207,7 @@ int mpdx_fused3d_planes_per_cta(int lx);
  * on the host, so a caller that captures mpdx_advance into a CUDA graph does so
  * after these 17 steps, or fixes the value with mpdx_fused3d_planes_per_cta), then the
  * fastest is kept for the handle's life.  chosen is 0 while tuning (or on a
- * handle that has not taken the fused 3D path); ms[] holds each candidate's time
+ * handle that does not take the fused 3D kernel); ms[] holds each candidate's time
  * per step once the choice is made. */
 typedef struct {
   int chosen;

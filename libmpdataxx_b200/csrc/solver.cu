@@ -284,11 +284,13 @@ struct mpdata_solver : solver_base {
   // of a chunk is mostly latency: 96^3 110 and 61, 160^3 112 and 200.  FP64 2D: three
   // passes 128^2 134 and 34, 1024^2 200 and 112, 4096^2 1476 and 1446; two passes 512^2
   // 43 and 26, 1024^2 44 and 47.  FP32 2D stays with the fused kernel, whose results
-  // equal the batched advance's bit for bit.
+  // equal the batched advance's bit for bit.  A process-wide setting of the fused kernel's
+  // planes holds for FP64 too, whose fields are the same bits either way; in FP32 they
+  // differ in rounding, so there the setting has no say in the choice.
   bool stages_faster() const {
     if (!stage_engine<T>::covers(st)) return false;
     const bool dbl = sizeof(T) == 8;
-    if (st.nd == 3) return dbl || (st.cells() <= 1000000 && fused3d_planes_setting(-1) == 0);
+    if (st.nd == 3) return dbl ? fused3d_planes_setting(-1) == 0 : st.cells() <= 1000000;
     return dbl && st.cells() <= (st.n_iters == 3 ? 16000000 : 600000);
   }
   bool line_cyclic() const {
@@ -367,7 +369,7 @@ struct mpdata_solver : solver_base {
   void tuning3d(mpdx_tuning3d *out) override {
     std::memset(out, 0, sizeof(*out));
     const int fixed = fused3d_planes_setting(-1);
-    out->chosen = fixed > 0 ? fixed : fus.lx3;
+    out->chosen = st.nd == 3 && path == MPDX_PATH_AUTO && stages_faster() ? 0 : (fixed > 0 ? fixed : fus.lx3);
     out->n_candidates = fused_engine<T>::kNumCand3;
     for (int q = 0; q < fused_engine<T>::kNumCand3; ++q) {
       out->lx[q] = fused_engine<T>::kCand3[q];

@@ -5,7 +5,7 @@ step; stats()["path"] names the path whose conditions the fields met, stats()["k
 the kernels that ran.  The fused kernels are run here with path="fused", whatever the
 automatic path would choose at the size: FP64 against the oracle to 1e-12, FP32 to 1e-5
 of the field's maximum, the bounds of the limiter exactly, bulk-tensor against
-per-thread plane copies bit for bit.  In FP64 3D the staged step
+per-thread plane copies and every chunk length bit for bit.  In FP64 3D the staged step
 gives the fused kernel's bits."""
 import numpy as np
 import pytest
@@ -109,3 +109,34 @@ def test_bulk_copies_bitwise(grid, opts):
     orc.advance(6)
     b = orc.advectee()
     assert np.abs(res[1].astype(np.float64) - b).max() <= 1e-5 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("grid,dtype,kernels", [(LARGE3, np.float64, FUSED), (LARGE3, np.float32, FUSED), (SMALL3, np.float64, FUSED),
+                                                (SMALL3, np.float32, STAGES)])
+def test_planes_setting(grid, dtype, kernels):
+    """On the automatic path: taken by the handles that the header names, the same fields
+    for every value, set before the run or between two advances."""
+    L, s, res = _lib.lib(), periodic_setup(grid, seed=23), []
+    try:
+        for lx in (64, 8, 512):
+            L.mpdx_fused3d_planes_per_cta(lx)
+            run, _ = run_both(s, o.iga | o.fct, 2, dtype, 0)
+            run.advance(4)
+            assert run.stats()["kernels"] == kernels
+            assert run.tuning3d()["chosen"] == (lx if kernels == FUSED else 0)
+            res.append(np.array(run.advectee()))
+        L.mpdx_fused3d_planes_per_cta(0)
+        run, _ = run_both(s, o.iga | o.fct, 2, dtype, 0)
+        run.advance(2)
+        L.mpdx_fused3d_planes_per_cta(96)
+        run.advance(2)
+        res.append(np.array(run.advectee()))
+        L.mpdx_fused3d_planes_per_cta(0)
+        run, _ = run_both(s, o.iga | o.fct, 2, dtype, 0)
+        run.advance(4)
+        assert run.tuning3d()["chosen"] == 0
+        res.append(np.array(run.advectee()))
+    finally:
+        L.mpdx_fused3d_planes_per_cta(0)
+    for a in res[1:]:
+        np.testing.assert_array_equal(a, res[0])
