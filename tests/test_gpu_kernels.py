@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 
 from libmpdataxx_b200 import _lib, opts as o
+from test_gpu_edges import NO_DIV, random_problem
 from test_gpu_fused import CASES_2D, CASES_3D, periodic_setup, run_both
 from test_gpu_parity import make_run, rel_err
 
@@ -140,3 +141,27 @@ def test_planes_setting(grid, dtype, kernels):
         L.mpdx_fused3d_planes_per_cta(0)
     for a in res[1:]:
         np.testing.assert_array_equal(a, res[0])
+
+
+C, O, R = "cyclic", "open", "rigid"
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("opts,iters", [(0, 1), (0, 3), (o.fct, 2), (o.fct, 3), (o.iga, 2), (o.iga | o.fct, 3),
+                                        (o.iga | o.tot | o.fct, 2), (o.tot, 3), (o.tot | o.fct, 3)])
+@pytest.mark.parametrize("grid,bcs", [((37,), [C, C]), ((37,), [O, O]), ((9, 13), [C, C, O, O]), ((11, 12), [O, R, R, O]),
+                                      ((70, 67), [R, R, C, C]), ((8, 9, 7), [C, C, O, O, R, R]), ((9, 7, 8), [R, O, C, C, O, O]),
+                                      ((6, 21, 69), [O, O, O, O, O, O])])
+def test_stages_equal_formulas(grid, bcs, opts, iters, dtype):
+    """The staged step gives the bits of one kernel per formula.  The latter is reached by an
+    option that changes nothing: in 1D and 3D fot, in 2D nug with its G of 1."""
+    s, out = random_problem(grid, seed=sum(grid) + iters), []
+    for extra, kernels in ((0, STAGES), (o.nug if len(grid) == 2 else o.fot, FORMULAS)):
+        run = make_run(grid, opts | extra, n_iters=iters, bcs=bcs, dtype=dtype, max_abs_div_eps=NO_DIV)
+        run.set_advectee(s["advectee"][0].astype(dtype))
+        for d, a in enumerate(s["advector"]):
+            run.set_advector(a.astype(dtype), d)
+        run.advance(3)
+        assert run.stats()["kernels"] == kernels
+        out.append(np.array(run.advectee()))
+    np.testing.assert_array_equal(*out)
