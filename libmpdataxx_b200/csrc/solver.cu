@@ -869,12 +869,10 @@ mpdx_status mpdx_get_field(mpdx_handle h, int kind, int idx, void *host, const i
   });
 }
 
-// the handle's stream waits for the work issued so far to the legacy default stream
-// (nothing to wait for when that has all ended: the query costs about 1 us, the event,
-// made once per handle, about 4)
+// the handle's stream waits for the work issued so far to the legacy default stream, by
+// an event made once per handle (one made for each call: 15.1 us per fetch in an ensemble
+// of 256 handles, with a query of that stream before it 14.8, so 13.4)
 static void after_legacy_stream(mpdx::solver_base &h) {
-  if (cudaStreamQuery(cudaStreamLegacy) == cudaSuccess) return;
-  (void)cudaGetLastError();
   if (!h.ev_legacy) MPDX_CUDA(cudaEventCreateWithFlags(&h.ev_legacy, cudaEventDisableTiming));
   MPDX_CUDA(cudaEventRecord(h.ev_legacy, cudaStreamLegacy));
   MPDX_CUDA(cudaStreamWaitEvent(h.stream, h.ev_legacy, 0));
