@@ -89,6 +89,14 @@ struct fld_axpy {
   __device__ __forceinline__ T operator()(long long q) const { return x[q] + b * y[q]; }
 };
 
+// the same through pointers that the bounds-checked build checks
+template <class T>
+struct ptr_axpy {
+  fptr<T> x, y;
+  T b;
+  __device__ __forceinline__ T operator()(long long q) const { return x[q] + b * y[q]; }
+};
+
 template <class T>
 __device__ __forceinline__ long long off3(const dfield<T> &f, int i, int j, int k) {
   return (long long)i * f.s0 + (long long)j * f.s1 + (long long)k * f.s2;
@@ -1008,7 +1016,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
   __syncthreads();
   rewind();
   if (R > 0) locate(first);
-  T *const phio = phi.o, *const leo = lap_err.o;
+  const auto phio = pointer(phi), leo = pointer(lap_err);
   T e[U], le[U], ph[U], po[U][K], lpo[U][K];
   bool alive = true;
   for (long long body = 0; body < max_bodies && !done && alive; ++body) {
@@ -1017,13 +1025,12 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
       const T b = den != T(0) ? -pnum / den : beta;  // beta keeps its value when tmp_den is 0
       beta = b;
       // first half: err' = err + beta lap_p_v, lap(err'), max |err'|, alpha sums
-      const T *const eao = cur ? err1.o : err0.o;
-      T *const ebo = cur ? err0.o : err1.o;
-      const T *lpv = D.lp[0].o;
+      const auto eao = cur ? pointer(err1) : pointer(err0), ebo = cur ? pointer(err0) : pointer(err1);
+      auto lpv = pointer(D.lp[0]);
 #pragma unroll
       for (int l = 0; l < K; ++l)
-        if (l == v) { tden[l] = den; lpv = D.lp[l].o; }
-      const fld_axpy<T> enew{eao, lpv, b};
+        if (l == v) { tden[l] = den; lpv = pointer(D.lp[l]); }
+      const ptr_axpy<T> enew{eao, lpv, b};
       dd acc[K];
 #pragma unroll
       for (int l = 0; l < K; ++l) acc[l] = dd{0.0, 0.0};
@@ -1038,8 +1045,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
 #pragma unroll
           for (int l = 0; l < K; ++l)
             if (l <= v) {
-              lpo[u][l] = D.lp[l].o[o[u]];
-              if (R > 0) po[u][l] = D.p[l].o[o[u]];
+              lpo[u][l] = elem(D.lp[l], o[u]);
+              if (R > 0) po[u][l] = elem(D.p[l], o[u]);
             }
           le[u] = lap_tab<T>(enew, g, sd, t_off, t_how, co[u], o[u], e[u]);
         }
@@ -1066,10 +1073,10 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
         if (l <= v && tden[l] != T(0)) alpha[l] = -T(ddv(acc[l])) / tden[l];
       // second half: Phi += beta p_v, next direction and its lap, beta sums
       const bool restart = v == K - 1;
-      T *pd = D.p[0].o, *lpd = D.lp[0].o;
+      auto pd = pointer(D.p[0]), lpd = pointer(D.lp[0]);
 #pragma unroll
       for (int l = 1; l < K; ++l)
-        if (!restart && l == v + 1) { pd = D.p[l].o; lpd = D.lp[l].o; }
+        if (!restart && l == v + 1) { pd = pointer(D.p[l]); lpd = pointer(D.lp[l]); }
       dd bs[2] = {{0.0, 0.0}, {0.0, 0.0}};
       auto second = [&](int oo, T ev, T lv, T pv, const T (&pp)[K], const T (&lp)[K]) {
         T pn = ev, ln = lv;
@@ -1103,7 +1110,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
             pv[u] = phio[oo[u]];
 #pragma unroll
             for (int l = 0; l < K; ++l)
-              if (l <= v) { pp[u][l] = D.p[l].o[oo[u]]; lp[u][l] = D.lp[l].o[oo[u]]; }
+              if (l <= v) { pp[u][l] = elem(D.p[l], oo[u]); lp[u][l] = elem(D.lp[l], oo[u]); }
           }
 #pragma unroll
           for (int u = 0; u < W; ++u)
@@ -1431,8 +1438,8 @@ __global__ void __launch_bounds__(256) k_advector(geom g, const gc_args<T> A) {
     const long long os = off3(st, c[0], c[1], c[2]), ou = off3(ve, c[0], c[1], c[2]);
     const long long ss = stride(st, d), su = stride(ve, d);
     auto at = [&](int q) {
-      T s = st.o[os + q * ss] * -A.b;
-      s = s + (T(1) + A.b) * ve.o[ou + q * su];
+      T s = elem(st, os + q * ss) * -A.b;
+      s = s + (T(1) + A.b) * elem(ve, ou + q * su);
       return s;
     };
     const int n = g.n[d];
@@ -1441,7 +1448,7 @@ __global__ void __launch_bounds__(256) k_advector(geom g, const gc_args<T> A) {
       if (q > n - 1) return T(2) * at(n - 1) - at(2 * (n - 1) - q);
       return at(q);
     };
-    gc.o[to] = A.c[d] * (filled(f) + filled(f + 1));
+    elem(gc, to) = A.c[d] * (filled(f) + filled(f + 1));
   }
 }
 

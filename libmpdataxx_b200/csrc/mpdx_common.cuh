@@ -119,6 +119,58 @@ struct dfield {
   }
 };
 
+// where linear offset q from element (0, 0, 0) lies, by the layout of field<T>::alloc
+// (rows of the last axis with `front` slots before index 0, a whole number of 128-byte
+// lines; rows of a plane as many as axis 1 has indices)
+#ifdef MPDX_BOUNDS_CHECK
+template <class T>
+__host__ __device__ inline void index_of(const dfield<T> &f, long long q, long long (&c)[3]) {
+  constexpr long long align = 128 / sizeof(T);
+  const int last = f.s2 ? 2 : (f.s1 ? 1 : 0);
+  const long long front = (-f.lo[last] + align - 1) / align * align;
+  auto floor_div = [](long long a, long long b) { return a >= 0 ? a / b : -((-a + b - 1) / b); };
+  c[0] = c[1] = c[2] = 0;
+  if (last == 0) { c[0] = q; return; }
+  const long long pitch = last == 2 ? f.s1 : f.s0, row = floor_div(q + front, pitch);
+  c[last] = q - row * pitch;
+  if (last == 1) { c[0] = row; return; }
+  const long long rows = f.s0 / f.s1;
+  c[0] = floor_div(row - f.lo[1], rows);
+  c[1] = row - c[0] * rows;
+}
+template <class T>
+__device__ __noinline__ T &checked(const dfield<T> &f, long long q) {
+  if (!f.oob || f.lo[0] > f.hi[0]) return f.o[q];
+  long long c[3];
+  index_of(f, q, c);
+  auto in = [](long long x) { return int(x < -(1LL << 30) ? -(1LL << 30) : (x > (1LL << 30) ? 1LL << 30 : x)); };
+  return f(in(c[0]), in(c[1]), in(c[2]));
+}
+#endif
+// the element at linear offset q of a field, and a pointer that walks a field: plain
+// addresses, which the bounds-checked build checks like operator()
+template <class T>
+__device__ __forceinline__ T &elem(const dfield<T> &f, long long q) {
+#ifdef MPDX_BOUNDS_CHECK
+  return checked(f, q);
+#else
+  return f.o[q];
+#endif
+}
+#ifdef MPDX_BOUNDS_CHECK
+template <class T>
+struct fptr {
+  dfield<T> f;
+  long long q;
+  __device__ __forceinline__ T &operator[](long long i) const { return elem(f, q + i); }
+  __host__ __device__ __forceinline__ fptr operator+(long long i) const { return {f, q + i}; }
+};
+template <class T> __host__ __device__ __forceinline__ fptr<T> pointer(const dfield<T> &f) { return {f, 0}; }
+#else
+template <class T> using fptr = T *;
+template <class T> __host__ __device__ __forceinline__ T *pointer(const dfield<T> &f) { return f.o; }
+#endif
+
 // Owning device allocation of one field (scalar, or one vector component).
 // The fastest-varying dimension is padded so that index 0 of every row sits on
 // a 128-byte boundary; rows have a pitch that is a multiple of 128 bytes.

@@ -26,7 +26,7 @@ namespace mpdx {
 // rows of any alignment.  Bound by DRAM (8.4 M FP32 elements: 61 us with one element
 // per thread found by two 64-bit divisions).
 template <class T>
-__global__ void __launch_bounds__(256) k_view_copy(T *f, long long s0, long long s1, T *buf, int rows, int n1, int n, bool to_field) {
+__global__ void __launch_bounds__(256) k_view_copy(fptr<T> f, long long s0, long long s1, T *buf, int rows, int n1, int n, bool to_field) {
   const int nseg = (n + 127) >> 7;
   const long long tot = (long long)rows * nseg;
   const int lane = threadIdx.x & 31;
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(256) k_view_copy(T *f, long long s0, long long
     const int row = tot <= 0x7fffffff ? int(unsigned(q) / unsigned(nseg)) : int(q / nseg);
     const int c0 = int(q - (long long)row * nseg) * 128 + lane;
     const int a = row / n1;
-    T *const x = f + a * s0 + (row - a * n1) * s1;
+    const auto x = f + (a * s0 + (row - a * n1) * s1);
     T *const y = buf + (long long)row * n;
     T v[4];
 #pragma unroll
@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(256) k_view_copy(T *f, long long s0, long long
       if (c0 + 32 * u < n) v[u] = to_field ? y[c0 + 32 * u] : x[c0 + 32 * u];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (c0 + 32 * u < n) (to_field ? x : y)[c0 + 32 * u] = v[u];
+      if (c0 + 32 * u < n) (to_field ? x[c0 + 32 * u] : y[c0 + 32 * u]) = v[u];
   }
 }
 // the view ex at offset off of field f (C order in buf)
@@ -53,7 +53,7 @@ void view_copy(cudaStream_t s, const field<T> &f, T *buf, const int ex[3], const
   const int n1 = f.nd == 3 ? ex[1] : 1, rows = f.nd == 1 ? 1 : ex[0] * n1;
   const long long segs = (long long)rows * ((n + 127) / 128);
   if (segs <= 0) return;
-  T *const o = f.v.o + off[0] * f.v.s0 + off[1] * f.v.s1 + off[2] * f.v.s2;
+  const auto o = pointer(f.v) + (off[0] * f.v.s0 + off[1] * f.v.s1 + off[2] * f.v.s2);
   k_view_copy<T><<<unsigned(std::min<long long>((segs + 7) / 8, 148 * 32)), 256, 0, s>>>(o, f.v.s0, f.v.s1, buf, rows, n1, n, to_field);
   MPDX_LAUNCH_CHECK();
 }

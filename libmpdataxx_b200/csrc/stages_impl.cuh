@@ -55,7 +55,7 @@ template <class T> __device__ __forceinline__ T div6(T x) { return qdiv<T>(x, T(
 // a field by 32-bit element strides
 template <class T>
 struct arr {
-  T *o;
+  fptr<T> o;
   int s0, s1;  // strides of axes 0 and 1 (the last axis: 1)
 };
 
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::upwind) k_upwind(con
     int c[3];
     if (!own<ND>(A, c)) return;
     after_previous();
-    const T *p = E.in.o, *g = E.unco[0].o;
+    const auto p = E.in.o, g = E.unco[0].o;
     const T p0 = p[c[0]], pp = p[src(A, 0, c[0] + 1)], pm = p[src(A, 0, c[0] - 1)], g1 = g[c[0]], g0 = g[c[0] - 1];
     const T nt = net(A, 0, c[0], [&](int f) { return f == 0 ? flux(g1, p0, pp) : flux(g0, pm, p0); });
     E.out.o[c[0]] = p0 + nt;
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::upwind) k_upwind(con
     T lo = flux(plane(F0, w.i0 - 1)[a0], plane(E.in, src(A, 0, w.i0 - 1))[o], p0);
 #pragma unroll 2
     for (int i = w.i0; i < w.i1; ++i) {
-      const T *q = plane(E.in, i), *q1 = plane(F1, i);
+      const auto q = plane(E.in, i), q1 = plane(F1, i);
       const T pn = plane(E.in, src(A, 0, i + 1))[o], g0 = plane(F0, i)[a0];
       const T pj = q[oj], pjm = q[ojm], g1 = q1[a1], g1m = q1[a1 - s1];
       T nt[3];
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::upwind) k_upwind(con
       nt[0] = net(A, 0, i, [&](int f) { return f == 0 ? hi : lo; });
       nt[1] = net(A, 1, j, [&](int f) { return f == 0 ? flux(g1, p0, pj) : flux(g1m, pjm, p0); });
       if constexpr (ND == 3) {
-        const T *q2 = plane(F2, i);
+        const auto q2 = plane(F2, i);
         const T pk = q[ok], pkm = q[okm], g2 = q2[a2], g2m = q2[a2 - 1];
         nt[2] = net(A, 2, k, [&](int f) { return f == 0 ? flux(g2, p0, pk) : flux(g2m, pkm, p0); });
       }
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::antidiff) k_antidiff
     auto plane = [&](const arr<T> &f, int i) { return f.o + (long long)i * f.s0; };
     T P[3][3][3], g0c, g0j, g0k = T(0), h1 = T(0), h1m = T(0), h2 = T(0), h2m = T(0);
     auto load = [&](T (&Q)[3][3], int i) {
-      const T *q = plane(E.in, src(A, 0, i));
+      const auto q = plane(E.in, src(A, 0, i));
 #pragma unroll
       for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -402,13 +402,13 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::antidiff) k_antidiff
     load(P[0], w.i0 - 1);
     load(P[1], w.i0);
     {
-      const T *q = plane(F0, w.i0 - 1);
+      const auto q = plane(F0, w.i0 - 1);
       g0c = q[a0];
       g0j = zj ? T(0) : q[a0j];
       if (ND == 3) g0k = zk ? T(0) : q[a0k];
-      const T *r = plane(F1, w.i0);
+      const auto r = plane(F1, w.i0);
       h1 = r[a1]; h1m = r[a1 - s1];
-      if (ND == 3) { const T *t = plane(F2, w.i0); h2 = t[a2]; h2m = t[a2 - 1]; }
+      if (ND == 3) { const auto t = plane(F2, w.i0); h2 = t[a2]; h2m = t[a2 - 1]; }
     }
 #pragma unroll 2
     for (int i = w.i0; i < w.i1; ++i) {
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::antidiff) k_antidiff
       int iv = i + 1;
       bool zi = false;
       if (!HALO) zi = !vsrc(A, 0, iv);
-      const T *q0 = plane(F0, i), *q1 = plane(F1, i), *n1 = plane(F1, iv), *q2 = plane(F2, i), *n2 = plane(F2, iv);
+      const auto q0 = plane(F0, i), q1 = plane(F1, i), n1 = plane(F1, iv), q2 = plane(F2, i), n2 = plane(F2, iv);
       const T c0 = q0[a0], c0j = zj ? T(0) : q0[a0j];
       T c0k = T(0), c1k = T(0), c1km = T(0), c2j = T(0), c2jm = T(0), m2 = T(0), m2m = T(0);
       const T m1 = zi ? T(0) : n1[a1], m1m = zi ? T(0) : n1[a1 - s1];
@@ -626,18 +626,18 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::betas) k_betas(const
 #pragma unroll 2
     for (int i = w.i0; i < w.i1; ++i) {
       const int ip = src(A, 0, i + 1);
-      const T *p = plane(E.in, i), *f1 = plane(F1, i);
+      const auto p = plane(E.in, i), f1 = plane(F1, i);
       const T pn = plane(E.in, ip)[o], c1 = plane(F0, i)[a0];
       T ph[3], pl[3], hi[3], lo[3];
       ph[0] = pn; pl[0] = pm; hi[0] = c1; lo[0] = c0;
       ph[1] = p[oj]; pl[1] = p[ojm]; hi[1] = f1[a1]; lo[1] = f1[a1 - s1];
-      if (ND == 3) { const T *f2 = plane(F2, i); ph[2] = p[ok]; pl[2] = p[okm]; hi[2] = f2[a2]; lo[2] = f2[a2 - 1]; }
+      if (ND == 3) { const auto f2 = plane(F2, i); ph[2] = p[ok]; pl[2] = p[okm]; hi[2] = f2[a2]; lo[2] = f2[a2 - 1]; }
       const long long oc = (long long)i * E.bu.s0 + o;  // the limiters have the layout of psi
       T mn, mx, qn = T(0);
       if (MODE == 2) {
         mn = E.mn.o[oc]; mx = E.mx.o[oc];
       } else {
-        const T *q = plane(E.psin, i);
+        const auto q = plane(E.psin, i);
         qn = plane(E.psin, ip)[o];
         T h[3] = {qn, q[oj], T(0)}, l[3] = {qm, q[ojm], T(0)};
         if (ND == 3) { h[2] = q[ok]; l[2] = q[okm]; }
@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::correct) k_correct(c
     if (!own<ND>(A, c)) return;
     after_previous();
     const int x = c[0];
-    const T *p = E.in.o, *f = E.corr[0].o, *bu = E.bu.o, *bd = E.bd.o;
+    const auto p = E.in.o, f = E.corr[0].o, bu = E.bu.o, bd = E.bd.o;
     T ch = f[x], cl = f[x - 1];
     if (FCT) {
       ch = limited(ch, bu[x], bd[x], bu[x + 1], bd[x + 1]);
@@ -696,12 +696,12 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::correct) k_correct(c
     if (!IGA) lo = flux(lo, plane(E.in, src(A, 0, w.i0 - 1))[o], p0);
 #pragma unroll 2
     for (int i = w.i0; i < w.i1; ++i) {
-      const T *q = plane(E.in, i), *f1 = plane(F1, i);
+      const auto q = plane(E.in, i), f1 = plane(F1, i);
       T pn = T(0), bun = T(0), bdn = T(0), hi = plane(F0, i)[a0];
       T yh = f1[a1], yl = f1[a1 - s1];
       if (!IGA || i + 1 < w.i1) pn = plane(E.in, src(A, 0, i + 1))[o];
       if (FCT) {
-        const T *u = plane(E.bu, i), *v = plane(E.bd, i);
+        const auto u = plane(E.bu, i), v = plane(E.bd, i);
         bun = plane(E.bu, i + 1)[o]; bdn = plane(E.bd, i + 1)[o];
         hi = limited(hi, bu0, bd0, bun, bdn);
         yh = limited(yh, bu0, bd0, u[o + sj], v[o + sj]);
@@ -712,10 +712,10 @@ __global__ void __launch_bounds__(kStageThreads, blocks<T>::correct) k_correct(c
       nt[0] = net(A, 0, i, [&](int f) { return f == 0 ? hi : lo; });
       nt[1] = net(A, 1, j, [&](int f) { return f == 0 ? yh : yl; });
       if constexpr (ND == 3) {
-        const T *f2 = plane(F2, i);
+        const auto f2 = plane(F2, i);
         T zh = f2[a2], zl = f2[a2 - 1];
         if (FCT) {
-          const T *u = plane(E.bu, i), *v = plane(E.bd, i);
+          const auto u = plane(E.bu, i), v = plane(E.bd, i);
           zh = limited(zh, bu0, bd0, u[o + 1], v[o + 1]);
           zl = limited(zl, u[o - 1], v[o - 1], bu0, bd0);
         }
@@ -746,9 +746,8 @@ __host__ __device__ constexpr int line_radius(int passes, bool fct, bool tot) {
 
 template <class T>
 struct line_args {
-  const T *in[kStageEqns];
-  T *out[kStageEqns];
-  const T *gc;  // faces -hv .. n-2+hv
+  fptr<T> in[kStageEqns], out[kStageEqns];
+  fptr<T> gc;  // faces -hv .. n-2+hv
   int n, steps, halo, hv;
   bool cyclic;
   long long t0;
@@ -776,8 +775,7 @@ __global__ void __launch_bounds__(128) k_line(const line_args<T> A) {
   const int x0 = seg * useful;
   if (x0 >= P) return;  // whole warps
   const int xs = x0 - A.halo;  // first point of the segment
-  const T *const in = A.in[blockIdx.y];
-  T *const out = A.out[blockIdx.y];
+  const auto in = A.in[blockIdx.y], out = A.out[blockIdx.y];
   next_may_start();
   after_previous();
   int x[4];
@@ -918,7 +916,7 @@ inline int planes_per_thread(int n0, long long blocks) {
 
 template <class T>
 arr<T> view(const field<T> &f) {
-  return {f.v.o, int(f.v.s0), int(f.v.s1)};
+  return {pointer(f.v), int(f.v.s0), int(f.v.s1)};
 }
 
 template <class T, int ND>
@@ -1042,7 +1040,7 @@ void stage_engine<T>::line(mpdata_state<T> &st, long long nt) {
     a.n = n;
     a.hv = st.H;
     a.cyclic = st.bcs[0][0] == MPDX_BC_CYCLIC;
-    a.gc = st.GC[0].v.o;
+    a.gc = pointer(st.GC[0].v);
     a.t0 = st.timestep;
     a.uff = st.upwind_filter_freq;
     const int useful = sg::kLinePoints - 2 * a.halo, bs = few ? 32 : 128;
@@ -1050,8 +1048,8 @@ void stage_engine<T>::line(mpdata_state<T> &st, long long nt) {
     for (int e0 = 0; e0 < st.n_eqns; e0 += kStageEqns) {
       const int ne = std::min(kStageEqns, st.n_eqns - e0);
       for (int q = 0; q < ne; ++q) {
-        a.in[q] = st.psi[e0 + q][st.tl[e0 + q]].v.o;
-        a.out[q] = st.psi[e0 + q][st.tl[e0 + q] ^ 1].v.o;
+        a.in[q] = pointer(st.psi[e0 + q][st.tl[e0 + q]].v);
+        a.out[q] = pointer(st.psi[e0 + q][st.tl[e0 + q] ^ 1].v);
         st.tl[e0 + q] ^= 1;
       }
       const dim3 g(ceil_div(segs, bs / 32), ne);
