@@ -803,6 +803,7 @@ void launch_inner(int v, unsigned G, dim3 blk, cudaStream_t s, const geom &g, in
 // step are latency-bound (rule and figures at loop_grid).  A wait that gives up after
 // about two seconds sets dv->timeout and leaves.
 constexpr int kLoopThreads = 512;
+constexpr long long kLoopWait = 1LL << 32;  // cycles: about two seconds
 
 // lap()'s index rules for every coordinate of an axis, in shared memory: element
 // offsets from the point to the neighbours of the two sides of the outer difference
@@ -871,7 +872,7 @@ __device__ __forceinline__ bool grid_wait(unsigned *bar, unsigned target, int *t
       if (int(v - target) >= 0) break;
       const long long t = clock64();
       if (t0 == 0) t0 = t;
-      if (t - t0 > (1LL << 32)) {
+      if (t - t0 > kLoopWait) {
         *reinterpret_cast<volatile int *>(timeout) = 1;
         ok = 0;
         break;

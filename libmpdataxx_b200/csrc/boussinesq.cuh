@@ -69,6 +69,19 @@ struct boussinesq {
   double2 *board = nullptr;    // partial sums of the one-launch loop's blocks, then the arrival counter
   int n_sm = 0;                // SMs (0: no cooperative launch)
   size_t board_bytes() const { return size_t(2) * kRedSlots * n_sm * sizeof(double2) + 128; }
+#ifdef MPDX_BOUNDS_CHECK
+  // (debug library) takes one arrival away, so that the next wait of the one-launch loop
+  // runs out
+  void lose_arrival() {
+    if (!board) throw error(MPDX_E_UNSUPPORTED, "no one-launch pressure solve on this device");
+    unsigned n = 0;
+    MPDX_CUDA(cudaMemcpyAsync(&n, board_bar(), sizeof(n), cudaMemcpyDeviceToHost, st.stream));
+    MPDX_CUDA(cudaStreamSynchronize(st.stream));
+    n -= 1;
+    MPDX_CUDA(cudaMemcpyAsync(board_bar(), &n, sizeof(n), cudaMemcpyHostToDevice, st.stream));
+    MPDX_CUDA(cudaStreamSynchronize(st.stream));
+  }
+#endif
   unsigned *board_bar() const { return reinterpret_cast<unsigned *>(board + size_t(2) * kRedSlots * n_sm) + 16; }
   int *vip_dev = nullptr;      // vip[] on the device
 

@@ -159,6 +159,9 @@ struct solver_base {
   virtual double precond_loss_grad(const double *, const double *, double, float *) {
     throw error(MPDX_E_UNSUPPORTED, "no pressure solve in this solver");
   }
+#ifdef MPDX_BOUNDS_CHECK
+  virtual void lose_arrival() { throw error(MPDX_E_UNSUPPORTED, "no pressure solve in this solver"); }
+#endif
   // the fused 3D kernel's chunk-length tuner (MPDATA solvers only)
   virtual void tuning3d(mpdx_tuning3d *out) { std::memset(out, 0, sizeof(*out)); }
 };
@@ -439,6 +442,9 @@ struct boussinesq_solver : solver_base {
     xfer.get(stream, *f, dst, device, ex, off);
   }
   void advance(long long nt) override { b->advance(nt); }
+#ifdef MPDX_BOUNDS_CHECK
+  void lose_arrival() override { b->lose_arrival(); }
+#endif
   void precond_record(long long n) override { b->precond_record(n); }
   double precond_train(long long steps, double lr, unsigned long long seed) override { return b->precond_train(steps, lr, seed); }
   void precond_enable(bool on) override { b->precond_enable(on); }
@@ -1079,6 +1085,14 @@ mpdx_status mpdx_precond_set_params(mpdx_handle h, const float *host) {
     h->impl->precond_params(nullptr, host);
   });
 }
+
+#ifdef MPDX_BOUNDS_CHECK
+// the debug library only: the next wait of the blocks of a one-launch pressure solve for
+// one another misses an arrival and gives up
+mpdx_status mpdx_debug_lose_arrival(mpdx_handle h) {
+  return guarded(h, [&] { h->impl->lose_arrival(); });
+}
+#endif
 
 void mpdx_destroy(mpdx_handle h) {
   if (!h) return;
