@@ -165,7 +165,10 @@ mpdx_status mpdx_get_field_async(mpdx_handle h, int kind, int idx, void *host);
 
 /* run.advance(nt)  (concurr_common.hpp:380-385 -> solver_common.hpp:270-358).
  * Asynchronous with respect to the host except on the first call (the
- * divergence check of hook_ante_loop reads one device scalar back). */
+ * divergence check of hook_ante_loop reads one device scalar back), on the first
+ * call after an upload where a periodic 2D or 3D problem may take the fused path (the
+ * check of its seams reads a flag back), on the steps of the fused 3D kernel's tuner
+ * and in Boussinesq solvers (the pressure solve's convergence). */
 mpdx_status mpdx_advance(mpdx_handle h, int64_t nt);
 
 /* Blocks until the handle's stream and its transfer streams are idle. */

@@ -5,7 +5,7 @@
 //   hook_ante_loop   mpdata_rhs_vip_prs_common.hpp:130-160 (initial projection,
 //                    ini_pressure), mpdata_rhs_vip_common.hpp:283-302, mpdata_rhs.hpp:154-169
 //   calc_gc          mpdata_rhs_vip_common.hpp:120-153 (extrp), mpdata_rhs_vip.hpp
-//                    (xchng_pres of the stash, intrp, advector halo fills)
+//                    (intrp and the halos around it): k_advector
 //   hook_ante_step   mpdata_rhs_vip_common.hpp:351-364, mpdata_rhs.hpp:171-193
 //   advection        general<T>::step() (solver_common.hpp:127-136)
 //   hook_post_step   mpdata_rhs.hpp:195-214, boussinesq_expl.hpp:83-126,
@@ -14,7 +14,8 @@
 //
 // Pointwise stages that the reference runs as separate array statements are
 // fused into one kernel each (the per-point arithmetic and its order are
-// unchanged).  The GCR iteration runs as two kernels per inner step:
+// unchanged).  The GCR iteration runs whole in one cooperative launch (k_gcr_loop) up to
+// 2.5 million points and k = 4 (loop_grid), else as two kernels per inner step:
 //   k_gcr_update: err' = err + beta lap_p_v, lap_err = lap(err'), max|err'| and
 //                 the alpha sums;
 //   k_gcr_direction: Phi += beta p_v (deferred here from the reference's first
@@ -27,8 +28,9 @@
 // rigid wall (set_edges), so no halo-fill kernels run inside the loop.  Sums
 // are compensated double-double reductions with a fixed tree (reproducible);
 // the last block of each reduction finalises the GCR scalars on the device.
-// Convergence is a device flag: bodies are launched in batches and kernels
-// return at once after convergence, so the host reads one flag per batch.
+// Convergence is a device flag: the one launch leaves when it is set; of the two
+// kernels, bodies are launched in batches and return at once after convergence, so the
+// host reads one flag per launch or batch.
 // Compiled with --fmad=false: FP64 results follow the reference's rounding.
 #include <algorithm>
 #include <cfloat>
@@ -1631,16 +1633,21 @@ unsigned red_grid(const bq::geom &g) {
 // shared planes of k_gcr_update3 save more than the launches cost, and axes that do
 // not fit the table of index rules.  FP64, us per iteration of cr, two launches
 // against one: 48 x 48 19 and 6.4, 201 x 201 22 (38 with whole rows per warp) and 7.2,
-// 400 x 400 32 and 10.8, 1000 x 1000 56 and 26, 97 x 89 x 65 53 and 20.6,
-// 128 x 128 x 96 67 and 42.6, 160 x 160 x 96 (2.46 M points) 89 and 73.5; gcrk with
-// k = 3 at 97 x 89 x 65 178 and 80.5 per body.  512 threads with 128 registers and two
+// 400 x 400 32 and 10.8, 1000 x 1000 56 and 26, 48^3 43 and 10.4, 97 x 89 x 65 53 and
+// 20.6, 128 x 128 x 96 68 and 42, 160 x 160 x 96 (2.46 M points) 89 and 73, 160 x 160 x 128
+// (3.28 M) 106 and 101, 192 x 192 x 128 (4.72 M) 128 and 144.  gcrk with k = 3, per body:
+// 97 x 89 x 65 178 and 80.5, 160 x 160 x 96 326 and 326, 192 x 192 x 128 486 and 593: the
+// line lies where k = 3 breaks even, below the 4 M or so of cr.  512 threads with 128 registers and two
 // points per pass: with 1024 threads and 64 registers fewer loads are in flight
 // (160 x 160 x 96: 120).
 struct loop_shape {
   int blocks, threads;
 };
 constexpr long long kLoopCells = 2500000;
-constexpr int kLoopMaxK = 4;  // longest basis built: longer ones spill (836 bytes for 8), and the library grows
+// longest basis built: longer ones spill more (836 bytes of stores per thread for 8; 24,
+// 104 and 120 for 2, 3 and 4 with several points per thread, none with one), and the
+// library grows
+constexpr int kLoopMaxK = 4;
 loop_shape loop_grid(const bq::geom &g, int n_sm, int k) {
   if (n_sm <= 0 || k > kLoopMaxK || g.cells > kLoopCells || g.n[0] + g.n[1] + (g.nd == 3 ? g.n[2] : 0) > bq::kLapRows) return {0, 0};
   const long long per_sm = (g.cells + n_sm - 1) / n_sm;

@@ -283,10 +283,14 @@ struct mpdata_solver : solver_base {
   // Where a step in stages (general<T>::step) beats the fused kernel on a periodic grid.
   // us per step, fused and stages.  FP64 3D always (the fused canvas of 16 x 64 computes
   // 1.83 points per result and is bound by FP64 issue): 24^3 168 and 25, 96^3 172 and
-  // 80, 250 x 257 x 241 1443 and 996, 400^3 5093 and 4535.  FP32 3D while the march
-  // of a chunk is mostly latency: 96^3 110 and 61, 160^3 112 and 200.  FP64 2D: three
-  // passes 128^2 134 and 34, 1024^2 200 and 112, 4096^2 1476 and 1446; two passes 512^2
-  // 43 and 26, 1024^2 44 and 47.  FP32 2D stays with the fused kernel, whose results
+  // 80, 250 x 257 x 241 1443 and 996, 400^3 5094 and 3988, 512^3 10494 and 8615.  FP32 3D
+  // while the march of a chunk is mostly latency: 96^3 110 and 47, 120^3 115 and 85,
+  // 140^3 114 and 122; the line, at 10^6 points, is on the safe side of that.  FP64 2D:
+  // three passes 128^2 134 and 34, 1024^2 200 and 112, 4000^2 1405 and 1297, 6000^2 3107
+  // and 2914, 8192^2 5464 and 5484; two passes 512^2 53 and 22, 774^2 53 and 36, 900^2 54
+  // and 45, 1024^2 54 and 51 (random fields; 44 and 47 on the rotation, whose zeros take
+  // the divisions' slow path): the lines stop where the gain is within what the data
+  // change.  FP32 2D stays with the fused kernel, whose results
   // equal the batched advance's bit for bit.  A process-wide setting of the fused kernel's
   // planes holds for FP64 too, whose fields are the same bits either way; in FP32 they
   // differ in rounding, so there the setting has no say in the choice.

@@ -143,7 +143,11 @@ constexpr int kStageThreads = 128;
 // Blocks per SM that the registers are kept for: the kernels wait on L2 and DRAM, and
 // the walk's carried values would otherwise leave 8 warps per SM (k_antidiff at 150
 // registers).  250 x 257 x 241 iga|fct, us per step without and with: FP64 1240 and 996,
-// FP32 657 and 633.
+// FP32 657 and 633.  The limits make most of the 3D kernels spill, which costs less than
+// the warps are worth.  Bytes stored and loaded per thread, FP64: k_upwind 40 / 96;
+// k_antidiff 4 / 4 (iga) to 176 / 252 (tot without iga); k_betas 40 / 68 to 64 / 108;
+// k_correct with the limiter 132 / 132 (iga), 268 / 408 (without); FP32: k_antidiff up to
+// 84 / 88 (iga|tot), k_correct 68 / 128.
 template <class T> struct blocks;
 template <> struct blocks<float> { static constexpr int upwind = 10, antidiff = 6, betas = 8, correct = 10; };
 template <> struct blocks<double> { static constexpr int upwind = 12, antidiff = 4, betas = 8, correct = 12; };
@@ -1065,7 +1069,12 @@ void stage_engine<T>::line(mpdata_state<T> &st, long long nt) {
 }
 
 // One launch takes up to kStageEqns equations of a small grid (their work arrays
-// together stay in cache and the launches count), one of a large grid.
+// together stay in cache and the launches count), one of a large grid.  Open, iga|fct,
+// FP64, four equations, us per step one by one and together: 101^2 62 and 16, 364 x 360
+// 52 and 26, 64^3 130 and 85, 512^2 71 and 40; above the line the gain goes on but
+// falls (724^2 101 and 82, 80^3 195 and 161, 1024^2 167 and 159) while the further work
+// arrays (10 fields per equation in 3D) grow, and no size lost: the line keeps them
+// to about 100 MB.
 constexpr long long kStageBatchCells = 1 << 18;
 
 // The further work arrays are made by the first step that has a use for them.  A step
