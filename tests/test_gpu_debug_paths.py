@@ -1,7 +1,7 @@
 """The kernels that walk fields by pointers, in the bounds-checked and NaN-poisoned build
 (MPDX_LIBRARY=debug, a separate process): staged step, several 1D steps per launch,
-Boussinesq step with its one-launch pressure solve, refilled advector halos, field views.
-They finish without an access outside a field and without NaN, and equal the oracle."""
+Boussinesq step with its one-launch pressure solve, refilled advector halos, field views;
+and the fused kernels, for the NaN.  They finish without an access outside a field and without NaN, and equal the oracle."""
 import json
 import os
 import subprocess
@@ -63,7 +63,16 @@ for grid, opts, iters in [((24, 22, 41), o.iga | o.fct, 2), ((40, 51), o.fct, 3)
         orc.advance(2)
         got = np.array(run.advectee())
         out.append([str(grid) + str(k), run.stats()["kernels"], bool(np.isfinite(got).all()), rel(got, orc.advectee())])
-for opts in (0, o.iga | o.fct):
+# the fused kernels by name, and the one-block 1D steps: nothing that was not written is read
+for grid, opts, iters in [((24, 22, 41), o.iga | o.fct, 2), ((24, 22, 41), o.fct, 2), ((23, 19), o.iga | o.fct, 2), ((40, 51), o.fct, 3)]:
+    s = periodic_setup(grid, seed=5)
+    run, orc = make_run(grid, opts, n_iters=iters, max_abs_div_eps=1e-6, path="fused"), Oracle(grid, opts, n_iters=iters, max_abs_div_eps=1e-6)
+    for r in (run, orc):
+        load(r, s)
+        r.advance(3)
+    got = np.array(run.advectee())
+    out.append(["fused " + str(grid), run.stats()["kernels"], bool(np.isfinite(got).all()), rel(got, orc.advectee())])
+for opts in (0, o.iga | o.fct, o.abs):
     run, orc = make_run((40,), opts, path="auto"), Oracle((40,), opts)
     psi = np.random.default_rng(1).uniform(0.5, 2.0, 40)
     psi[-1] = psi[0]
@@ -95,9 +104,10 @@ def debug_process(script):
 
 
 def test_walking_kernels_run_clean():
-    stages, line = 2, 4
+    stages, fused, line, block = 2, 3, 4, 5
     for name, kernels, finite, err in debug_process(SCRIPT):
-        assert kernels == (line if name in ("(300,)", "40 0", "40 33") else stages), (name, kernels)
+        want = fused if name.startswith("fused") else line if name in ("(300,)", "40 0", "40 33") else block if name == "40 2" else stages
+        assert kernels == want, (name, kernels)
         assert finite, name
         assert err <= 1e-12, (name, err)
 
